@@ -181,3 +181,59 @@ def tolerance(case):
     """bf16 results over bf16 probabilities, rounding alone.  Against float32 throughout, calls show rel 2.3e-3 to 2.8e-3 and
     max 9e-3 to 1.8e-2; two correct implementations may be both that far off."""
     return {"rel": 1e-2, "max": 0.1}
+
+
+# Beyond this many (query, key) pairs over all heads the 64-bit scores take too long.
+_EXACT_PAIRS = 5e10
+
+
+def exact(case, seed):
+    """What ``run`` returns, in 64 bits from the same inputs: one head and a slice of the queries at a time."""
+    B, H, S, op = case["B"], case["H"], case["S"], case["op"]
+    total = case["Skv"] * case.get("steps", 1)
+    if float(B) * H * S * total > _EXACT_PAIRS:
+        return None
+    state = prepare(case, seed)
+    lens, f64 = _kv_len(case), torch.float64
+    q, scale = state["q"], D ** -0.5
+    if op == "ring":
+        k, v = (torch.cat(shards, dim=2) for shards in zip(*state["shards"]))
+    else:
+        k, v = state["k"], state["v"]
+    if op == "block":
+        cos, sin = (t.to(f64) for t in state["rope"])
+        half = case["rotary"] // 2
+
+        def finished(x, weight):
+            x = x.transpose(1, 2).to(f64)
+            x = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-5) * weight.to(f64)
+            head, rest = x[..., :2 * half], x[..., 2 * half:]
+            turned = torch.cat([-head[..., half:], head[..., :half]], -1)
+            return torch.cat([head * cos + turned * sin, rest], -1)
+
+        q, k, v = finished(q, state["weights"][0]), finished(k, state["weights"][1]), v.transpose(1, 2)
+    elif op == "fp8":
+        def cast(x, by):
+            return (x.float() * by).clamp(-448, 448).to(torch.float8_e4m3fn)
+
+        q, k, scale = cast(q, scale / math.log(2)), cast(k, 1.0), math.log(2)
+    out = torch.zeros(B, H, S, D, dtype=f64, device="cuda")
+    table = _table(case) if op == "sparse" else None
+    rows = 256 if table else max(256, min(4096, int(3e8) // total))
+    for b in range(B):
+        last = min(lens[b], S) if S == case["Skv"] or op == "ring" else S
+        for h in range(H):
+            k64, v64 = k[b, h, :lens[b]].to(f64), v[b, h, :lens[b]].to(f64)
+            for lo in range(0, last, rows):
+                hi = min(lo + rows, last)
+                kk, vv = k64, v64
+                if table:
+                    tiles = torch.tensor(table[lo // 256], device="cuda")
+                    keys = (tiles[:, None] * 128 + torch.arange(128, device="cuda")).flatten()
+                    keys = keys[keys < lens[b]]
+                    kk, vv = k64[keys], v64[keys]
+                p = torch.softmax((q[b, h, lo:hi].to(f64) @ kk.T).mul_(scale), -1)
+                out[b, h, lo:hi] = p @ vv
+    if op == "block":
+        return out.transpose(1, 2).reshape(B, S, H * D) @ state["w_out"].to(f64)
+    return out
