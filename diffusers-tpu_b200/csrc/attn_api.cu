@@ -154,36 +154,47 @@ __global__ void __launch_bounds__(256) merge_pieces_kernel(const __grid_constant
 }
 
 // ---------------------------------------------------------------------------
-// Max L2 row norm per head of a bf16 [B,H,S,128] tensor (one warp per row),
-// folded into norms[h] with an integer atomic max (norms are non-negative).
+// Max L2 row norm per head of a bf16 [B,H,S,128] tensor, folded into norms[h] with an integer atomic max (norms are
+// non-negative).  One block per (chunk of rows, head, batch element); a warp reads a whole 256-byte row per load,
+// eight rows in flight, and the block ends in one atomic.  HBM-bound: the tensor is read once.  (Rows dealt to warps
+// over the whole tensor, each warp at another head with every row and so at a global atomic per row, took 130 us per
+// 113 MB tensor; a bounded-logit call on 2 x 24 x 4608 rows went from 708 to 487 us with this split.)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) row_norm_max_kernel(const __nv_bfloat16* __restrict__ x, int B, int H, int S,
-                                                           int64_t sb, int64_t sh, int64_t ss, float mult,
+constexpr int kNormRows = 256;         // rows of a block
+constexpr int kNormRowsInFlight = 8;   // per warp
+__global__ void __launch_bounds__(256) row_norm_max_kernel(const __nv_bfloat16* __restrict__ x, int S, int64_t sb,
+                                                           int64_t sh, int64_t ss, float mult,
                                                            float* __restrict__ norms) {
-  const int64_t rows = static_cast<int64_t>(B) * H * S;
-  const int lane = threadIdx.x & 31;
-  const int64_t warps_total = static_cast<int64_t>(gridDim.x) * 8;
-  float best = 0.f;
-  int best_h = -1;
-  for (int64_t rid = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5); rid < rows; rid += warps_total) {
-    // rows are visited head-major so one warp mostly stays inside one head
-    const int s = static_cast<int>(rid % S);
-    const int b = static_cast<int>((rid / S) % B);
-    const int h = static_cast<int>(rid / (static_cast<int64_t>(S) * B));
-    if (h != best_h) {
-      if (best_h >= 0 && lane == 0) atomicMax(reinterpret_cast<int*>(norms + best_h), __float_as_int(best));
-      best_h = h;
-      best = 0.f;
-    }
-    const uint2 raw = reinterpret_cast<const uint2*>(x + b * sb + h * sh + s * ss)[lane];
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-    const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-    float ss2 = a.x * a.x + a.y * a.y + c.x * c.x + c.y * c.y;
+  __shared__ float warp_best[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int h = blockIdx.y;
+  const __nv_bfloat16* base = x + blockIdx.z * sb + h * sh;
+  const int r0 = blockIdx.x * kNormRows, r1 = min(r0 + kNormRows, S);
+  float best = 0.f;                    // of the squared norms: rounding, square root and scaling are monotonic
+  for (int r = r0 + warp; r < r1; r += 8 * kNormRowsInFlight) {
+    uint2 raw[kNormRowsInFlight];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss2 += __shfl_xor_sync(0xffffffffu, ss2, o);
-    best = fmaxf(best, sqrtf(ss2) * mult);
+    for (int u = 0; u < kNormRowsInFlight; ++u) {
+      raw[u] = make_uint2(0u, 0u);
+      if (r + 8 * u < r1) raw[u] = reinterpret_cast<const uint2*>(base + (r + 8 * u) * ss)[lane];
+    }
+#pragma unroll
+    for (int u = 0; u < kNormRowsInFlight; ++u) {
+      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[u].x));
+      const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[u].y));
+      float ss2 = a.x * a.x + a.y * a.y + c.x * c.x + c.y * c.y;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss2 += __shfl_xor_sync(0xffffffffu, ss2, o);
+      best = fmaxf(best, ss2);
+    }
   }
-  if (best_h >= 0 && lane == 0) atomicMax(reinterpret_cast<int*>(norms + best_h), __float_as_int(best));
+  if (lane == 0) warp_best[warp] = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) best = fmaxf(best, warp_best[i]);
+    if (best > 0.f) atomicMax(reinterpret_cast<int*>(norms + h), __float_as_int(sqrtf(best) * mult));
+  }
 }
 
 __global__ void fixed_m_finish_kernel(const float* __restrict__ norms, int Hq, int Hkv, float gate,
@@ -665,13 +676,11 @@ extern "C" int dtb_fixed_m_operands(const dtb_attn_params* p, float gate, float*
   const float scale = p->scale > 0.f ? p->scale : 1.0f / sqrtf(static_cast<float>(p->D));
   // The reference takes the norm of the bf16-rounded product q * scale * log2(e); this kernel
   // applies the scale in f32 after the MMA, so the norm of the unrounded product is the exact bound.
-  auto blocks = [](int64_t rows) { return static_cast<unsigned>(std::min<int64_t>((rows + 7) / 8, 148 * 16)); };
-  row_norm_max_kernel<<<blocks(static_cast<int64_t>(p->B) * p->Hq * p->Sq), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(p->q), p->B, p->Hq, p->Sq, p->q_stride_b, p->q_stride_h, p->q_stride_s,
-      scale * kLog2e, norms);
-  row_norm_max_kernel<<<blocks(static_cast<int64_t>(p->B) * p->Hkv * p->Skv), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(p->k), p->B, p->Hkv, p->Skv, p->k_stride_b, p->k_stride_h, p->k_stride_s, 1.0f,
-      norms + p->Hq);
+  auto grid = [&](int H, int S) { return dim3((S + kNormRows - 1) / kNormRows, H, p->B); };
+  row_norm_max_kernel<<<grid(p->Hq, p->Sq), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(p->q), p->Sq, p->q_stride_b,
+                                                         p->q_stride_h, p->q_stride_s, scale * kLog2e, norms);
+  row_norm_max_kernel<<<grid(p->Hkv, p->Skv), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(p->k), p->Skv, p->k_stride_b,
+                                                           p->k_stride_h, p->k_stride_s, 1.0f, norms + p->Hq);
   fixed_m_finish_kernel<<<(p->Hq + 127) / 128, 128, 0, s>>>(norms, p->Hq, p->Hkv, gate, mk_out);
   return launch_ok("kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
 }
