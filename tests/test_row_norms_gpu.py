@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-import dtb200
+from dtb200 import ops
 
 pytestmark = pytest.mark.gpu
 
@@ -16,7 +16,7 @@ def test_row_norm_maxima_over_block_edges(S):
     q[1, 0, S - 1] *= 4
     q[0, 1, 0] *= 4
     k[1, 2, S - 1] *= 4
-    qn, kn = dtb200.row_norm_maxima(q, k)
+    qn, kn = ops.row_norm_maxima(q, k)
     mult = 128 ** -0.5 * 1.44269504
     want_q = q.double().norm(dim=-1).amax(dim=(0, 2)) * mult
     want_k = k.double().norm(dim=-1).amax(dim=(0, 2))
@@ -27,5 +27,5 @@ def test_row_norm_maxima_over_block_edges(S):
 
 def test_row_norm_maxima_of_zeros_are_zero():
     z = torch.zeros(1, 2, 300, 128, dtype=torch.bfloat16, device="cuda")
-    qn, kn = dtb200.row_norm_maxima(z, z)
+    qn, kn = ops.row_norm_maxima(z, z)
     assert qn.abs().max().item() == 0.0 and kn.abs().max().item() == 0.0
