@@ -10,6 +10,7 @@
 #include <cuda_fp8.h>
 
 #include "attn_kernel.cuh"
+#include "attn_solo.cuh"
 #include "host_common.h"
 
 namespace dtb {
@@ -303,6 +304,27 @@ constexpr int kMinPieceTiles = 4;      // no run shorter than this many key tile
 #endif
 constexpr int kPieceOverheadTiles = DTB_PIECE_OVERHEAD_TILES;
 
+// Key-tile times that a block costs beyond its key tiles: launch, pipeline fill and drain, epilogue.
+constexpr int kBlockOverheadTiles = 5;
+
+// Time of a launch with one CTA per block of `rows` query rows, in key-tile times.  A block with one query tile passes
+// two key tiles in the time of one.
+long long plain_time(const dtb_attn_params* p, int sms, int rows) {
+  const long long blocks = static_cast<long long>((p->Sq + rows - 1) / rows) * p->Hq * p->B;
+  const long long n = (p->Skv + kBlockN - 1) / kBlockN;
+  return (blocks + sms - 1) / sms * ((rows == kBlockM ? (n + 1) / 2 : n) + kBlockOverheadTiles);
+}
+
+// Whether `time` is worse than a launch of 128-row blocks.  Those read K and V once per 128 rows instead of once per
+// 256, which is paid for out of the margin: 108 blocks of 256 rows x 36 tiles take 68 us, about what 216 of 128 rows
+// would; 54 x 18 tiles take 35.2 us against 24.6 in 108 smaller blocks.
+bool solo_beats(const dtb_attn_params* p, int sms, long long time) { return 5 * plain_time(p, sms, kBlockM) < 4 * time; }
+
+bool solo_blocks(const dtb_attn_params* p) {
+  const int sms = current_sm_count();
+  return solo_beats(p, sms, plain_time(p, sms, kQTiles * kBlockM));
+}
+
 struct BalancedPlan {
   bool use = false;
   int slots = 0;
@@ -324,6 +346,8 @@ void plan_balanced(const dtb_attn_params* p, int sms, BalancedPlan* plan) {
   if (runs <= tail) return;
   const long long run_len = (tiles + runs - 1) / runs;
   if (run_len + kPieceOverheadTiles > n) return;   // the plain launch is as fast or faster
+  // ... and so may be 128-row blocks, where there are few blocks
+  if (solo_beats(p, sms, units / sms * (n + kBlockOverheadTiles) + run_len + kPieceOverheadTiles)) return;
   struct Piece { int x, tb, te; };
   Piece pieces[kMaxPieces];
   int np = 0;
@@ -393,31 +417,23 @@ cudaError_t ensure_kernel_attrs() {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && g_attrs_set[dev].load(std::memory_order_acquire)) return cudaSuccess;
-  e = cudaFuncSetAttribute(attn_fwd_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(kSmemBytes));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(attn_fwd_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(kSmemBytes));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(attn_fwd_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(kSmemBytes));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(attn_fwd_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(kSmemBytes));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(attn_fwd_pieces_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(kSmemBytes));
-  if (e != cudaSuccess) return e;
+  struct { const void* fn; size_t smem; } variants[] = {
+      {reinterpret_cast<const void*>(attn_fwd_kernel<false, false>), kSmemBytes},
+      {reinterpret_cast<const void*>(attn_fwd_kernel<true, false>), kSmemBytes},
+      {reinterpret_cast<const void*>(attn_fwd_kernel<false, true>), kSmemBytes},
+      {reinterpret_cast<const void*>(attn_fwd_kernel<true, true>), kSmemBytes},
+      {reinterpret_cast<const void*>(attn_fwd_pieces_kernel), kSmemBytes},
+      {reinterpret_cast<const void*>(attn_solo_kernel<false, false>), kSoloSmemBytes},
+      {reinterpret_cast<const void*>(attn_solo_kernel<true, false>), kSoloSmemBytes},
+      {reinterpret_cast<const void*>(attn_solo_kernel<false, true>), kSoloSmemBytes},
+      {reinterpret_cast<const void*>(attn_solo_kernel<true, true>), kSoloSmemBytes}};
   // The register hand-over inside the kernel (setmaxnreg) is sized for kLaunchRegs registers per thread at
   // launch; with any other count a warpgroup could wait for registers that never come.  Refuse to launch then.
-  const void* variants[5] = {reinterpret_cast<const void*>(attn_fwd_kernel<false, false>),
-                             reinterpret_cast<const void*>(attn_fwd_kernel<true, false>),
-                             reinterpret_cast<const void*>(attn_fwd_kernel<false, true>),
-                             reinterpret_cast<const void*>(attn_fwd_kernel<true, true>),
-                             reinterpret_cast<const void*>(attn_fwd_pieces_kernel)};
-  for (const void* fn : variants) {
+  for (const auto& v : variants) {
+    e = cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(v.smem));
+    if (e != cudaSuccess) return e;
     cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, fn);
+    e = cudaFuncGetAttributes(&fa, v.fn);
     if (e != cudaSuccess) return e;
     if (fa.numRegs != kLaunchRegs) return cudaErrorInvalidConfiguration;
   }
@@ -470,6 +486,17 @@ int fill_kernel_params(const dtb_attn_params* p, AttnKernelParams* kp) {
   kp->table_qblocks = 0;
   kp->table_width = 0;
   return DTB_OK;
+}
+
+// One CTA per query block, with 256-row blocks or (solo_blocks) 128-row ones.
+template <bool kResidual, bool kQkFp8>
+int launch_plain(const dtb_attn_params* p, const AttnKernelParams& kp, cudaStream_t s) {
+  if (solo_blocks(p)) {
+    attn_solo_kernel<kResidual, kQkFp8><<<dim3((p->Sq + kBlockM - 1) / kBlockM, p->Hq, p->B), dim3(kNumThreads), kSoloSmemBytes, s>>>(kp);
+  } else {
+    attn_fwd_kernel<kResidual, kQkFp8><<<dim3(q_blocks(p), p->Hq, p->B), dim3(kNumThreads), kSmemBytes, s>>>(kp);
+  }
+  return launch_ok("attn_fwd_kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
 }
 
 // Sweep with the last wave in pieces, then the merge (see plan_balanced).  `workspace` holds
@@ -581,8 +608,7 @@ extern "C" int dtb_attn_fwd(const dtb_attn_params* p, void* workspace, size_t wo
       if (workspace == nullptr || workspace_bytes < balanced_workspace_bytes(plan.slots)) plan.use = false;
     }
     if (plan.use) return launch_balanced(p, kp, plan, workspace, s);
-    attn_fwd_kernel<false, false><<<dim3(q_blocks(p), p->Hq, p->B), dim3(kNumThreads), kSmemBytes, s>>>(kp);
-    return launch_ok("kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
+    return launch_plain<false, false>(p, kp, s);
   }
 
   int splits = resolve_splits(p);
@@ -598,14 +624,9 @@ extern "C" int dtb_attn_fwd(const dtb_attn_params* p, void* workspace, size_t wo
   if (p->flags & DTB_FLAG_QK_FP8) {
     // E4M3 q/k: one kernel variant, no split-KV
     if (p->num_splits > 1) return DTB_ERR_UNSUPPORTED;
-    attn_fwd_kernel<false, true><<<dim3(q_blocks(p), p->Hq, p->B), block, kSmemBytes, s>>>(kp);
-    return launch_ok("kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
+    return launch_plain<false, true>(p, kp, s);
   }
-  if (splits == 1) {
-    const dim3 grid(q_blocks(p), p->Hq, p->B);
-    attn_fwd_kernel<false, false><<<grid, block, kSmemBytes, s>>>(kp);
-    return launch_ok("kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
-  }
+  if (splits == 1) return launch_plain<false, false>(p, kp, s);
   const size_t rows = static_cast<size_t>(splits) * p->B * p->Hq * p->Sq;
   kp.acc_o = static_cast<float*>(workspace);
   kp.acc_m = kp.acc_o + rows * kHeadDim;
@@ -639,12 +660,8 @@ extern "C" int dtb_attn_fwd_residual(const dtb_attn_params* p, const dtb_attn_re
   kp.q_offset = r->q_offset;
   kp.acc_init = r->init ? 1 : 0;
   kp.zero_padded_rows = 0;  // padded rows are zeroed by dtb_attn_finalize
-  const dim3 grid(q_blocks(p), p->Hq, p->B);
-  if (p->flags & DTB_FLAG_QK_FP8)
-    attn_fwd_kernel<true, true><<<grid, dim3(kNumThreads), kSmemBytes, static_cast<cudaStream_t>(stream)>>>(kp);
-  else
-    attn_fwd_kernel<true, false><<<grid, dim3(kNumThreads), kSmemBytes, static_cast<cudaStream_t>(stream)>>>(kp);
-  return launch_ok("kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
+  if (p->flags & DTB_FLAG_QK_FP8) return launch_plain<true, true>(p, kp, static_cast<cudaStream_t>(stream));
+  return launch_plain<true, false>(p, kp, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int dtb_attn_finalize(const dtb_attn_params* p, const dtb_attn_residual* r, void* stream) {
@@ -748,10 +765,7 @@ extern "C" int dtb_attn_fwd_static_scratch(const dtb_attn_params* p, void* strea
   if (st != DTB_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const dim3 block(kNumThreads);
-  if (splits == 1) {
-    attn_fwd_kernel<false, false><<<dim3(q_blocks(p), p->Hq, p->B), block, kSmemBytes, s>>>(kp);
-    return launch_ok("attn_fwd_kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
-  }
+  if (splits == 1) return launch_plain<false, false>(p, kp, s);
   const size_t rows = static_cast<size_t>(splits) * p->B * p->Hq * p->Sq;
   kp.acc_o = static_cast<float*>(scratch);
   kp.acc_m = kp.acc_o + rows * kHeadDim;
@@ -796,9 +810,7 @@ extern "C" int dtb_attn_fwd_scatter(const dtb_attn_params* p, const dtb_attn_sca
     if (plan.use && sc->workspace_bytes >= balanced_workspace_bytes(plan.slots))
       return launch_balanced(p, kp, plan, sc->workspace, static_cast<cudaStream_t>(stream));
   }
-  attn_fwd_kernel<false, false><<<dim3(q_blocks(p), p->Hq, p->B), dim3(kNumThreads), kSmemBytes,
-                           static_cast<cudaStream_t>(stream)>>>(kp);
-  return launch_ok("attn_fwd_kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
+  return launch_plain<false, false>(p, kp, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int dtb_scatter_heads(const dtb_scatter_heads_params* sp, void* stream) {
@@ -851,9 +863,7 @@ extern "C" int dtb_attn_fwd_sparse(const dtb_attn_params* p, const dtb_block_tab
   kp.head_class = tb->n_classes > 1 ? tb->head_class : nullptr;
   kp.table_qblocks = tb->q_blocks;
   kp.table_width = tb->width;
-  attn_fwd_kernel<false, false><<<dim3(q_blocks(p), p->Hq, p->B), dim3(kNumThreads), kSmemBytes,
-                           static_cast<cudaStream_t>(stream)>>>(kp);
-  return launch_ok("attn_fwd_kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
+  return launch_plain<false, false>(p, kp, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------------------------

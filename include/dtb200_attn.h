@@ -143,7 +143,8 @@ size_t dtb_attn_workspace_bytes(const dtb_attn_params* p);
  * units - numbered query block fastest, then head, then batch - are swept whole, one CTA each; when n_pieces > 0 the
  * remaining tail_units units are swept in n_pieces pieces, piece i being key tiles [tile_begin[i], tile_end[i]) of unit
  * unit[i], listed longest first; a piece with slot[i] >= 0 leaves its state in that scratch slot for the merge, and
- * the slots of one unit are consecutive in key order.  n_pieces == 0 means the plain launch.  The plan depends only
+ * the slots of one unit are consecutive in key order.  n_pieces == 0 means the plain launch, one CTA per unit or, where
+ * that leaves SMs idle, one per 128-row half of a unit.  The plan depends only
  * on the static shape; it plays the role of the reference's per-shape tile resolution, which logs one line per
  * resolved shape (diffusers_tpu/kernels/mesh_attention.py:199-216, diffusers_tpu/kernels/block_sizes.py:442-577). */
 #define DTB_MAX_PIECES 304
