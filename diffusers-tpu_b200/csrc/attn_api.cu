@@ -316,8 +316,8 @@ long long plain_time(const dtb_attn_params* p, int sms, int rows) {
 }
 
 // Whether `time` is worse than a launch of 128-row blocks.  Those read K and V once per 128 rows instead of once per
-// 256, which is paid for out of the margin: 108 blocks of 256 rows x 36 tiles take 68 us, about what 216 of 128 rows
-// would; 54 x 18 tiles take 35.2 us against 24.6 in 108 smaller blocks.
+// 256, which is paid for out of the margin: 144 blocks of 128 rows x 131 tiles take 187 us, 2.6 us per period, where a
+// period of 256-row blocks takes 1.6 to 1.9 us.  (54 blocks of 256 rows x 18 tiles: 35.2 us; 108 of 128 rows: 24.6 us.)
 bool solo_beats(const dtb_attn_params* p, int sms, long long time) { return 5 * plain_time(p, sms, kBlockM) < 4 * time; }
 
 bool solo_blocks(const dtb_attn_params* p) {
