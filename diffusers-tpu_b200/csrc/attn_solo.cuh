@@ -326,14 +326,18 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     for (int j = 0; j < n_own && ok; ++j) {
       const int e = 2 * j + t;
       // One thread checks that V_e and K_{e+2} have landed; its arrival on the P barriers carries that to the issuer.
-      bool kv_ok = true;
-      if (row_in_tile == 0) {
+      // It does so after the wait for S(e), not before: a parity wait for one use of a ring slot also returns while
+      // the use before it is still in flight, so that use has to be known complete.  V_e follows K_{e-1} in its slot
+      // (the last V follows V_{n-4}), which the other group checked for its P(e-3), and that group may be a tile behind;
+      // but S(e) is issued after P(e-3) V_{e-3}.  K_{e+2} follows V_{e-2}, which this thread checked itself.
+      bool landed = mbar_wait(smem_u32(&bars->s_full[t]), j & 1, ctx, SITE_S_FULL + t);
+      if (landed && row_in_tile == 0) {
         const int iv = place_v(e), ik = place_k(e + 2);
-        kv_ok = mbar_wait(smem_u32(&bars->kv_full[iv % kSoloStages]), (iv / kSoloStages) & 1, ctx, SITE_KV_FULL + iv % kSoloStages);
-        if (kv_ok && e + 2 < n_tiles)
-          kv_ok = mbar_wait(smem_u32(&bars->kv_full[ik % kSoloStages]), (ik / kSoloStages) & 1, ctx, SITE_KV_FULL + ik % kSoloStages);
+        landed = mbar_wait(smem_u32(&bars->kv_full[iv % kSoloStages]), (iv / kSoloStages) & 1, ctx, SITE_KV_FULL + iv % kSoloStages);
+        if (landed && e + 2 < n_tiles)
+          landed = mbar_wait(smem_u32(&bars->kv_full[ik % kSoloStages]), (ik / kSoloStages) & 1, ctx, SITE_KV_FULL + ik % kSoloStages);
       }
-      ok = __all_sync(0xffffffffu, kv_ok && mbar_wait(smem_u32(&bars->s_full[t]), j & 1, ctx, SITE_S_FULL + t));
+      ok = __all_sync(0xffffffffu, landed);
       if (!ok) break;
       tc_fence_after();
       const int tile = tile_list != nullptr ? tile_list[e] : e;
