@@ -320,10 +320,7 @@ long long plain_time(const dtb_attn_params* p, int sms, int rows) {
 // period of 256-row blocks takes 1.6 to 1.9 us.  (54 blocks of 256 rows x 18 tiles: 35.2 us; 108 of 128 rows: 24.6 us.)
 bool solo_beats(const dtb_attn_params* p, int sms, long long time) { return 5 * plain_time(p, sms, kBlockM) < 4 * time; }
 
-bool solo_blocks(const dtb_attn_params* p) {
-  const int sms = current_sm_count();
-  return solo_beats(p, sms, plain_time(p, sms, kQTiles * kBlockM));
-}
+bool solo_blocks(const dtb_attn_params* p, int sms) { return solo_beats(p, sms, plain_time(p, sms, kQTiles * kBlockM)); }
 
 struct BalancedPlan {
   bool use = false;
@@ -491,11 +488,11 @@ int fill_kernel_params(const dtb_attn_params* p, AttnKernelParams* kp) {
 // One CTA per query block, with 256-row blocks or (solo_blocks) 128-row ones.
 template <bool kResidual, bool kQkFp8>
 int launch_plain(const dtb_attn_params* p, const AttnKernelParams& kp, cudaStream_t s) {
-  if (solo_blocks(p)) {
+  if (solo_blocks(p, current_sm_count())) {
     attn_solo_kernel<kResidual, kQkFp8><<<dim3((p->Sq + kBlockM - 1) / kBlockM, p->Hq, p->B), dim3(kNumThreads), kSoloSmemBytes, s>>>(kp);
-  } else {
-    attn_fwd_kernel<kResidual, kQkFp8><<<dim3(q_blocks(p), p->Hq, p->B), dim3(kNumThreads), kSmemBytes, s>>>(kp);
+    return launch_ok("attn_solo_kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
   }
+  attn_fwd_kernel<kResidual, kQkFp8><<<dim3(q_blocks(p), p->Hq, p->B), dim3(kNumThreads), kSmemBytes, s>>>(kp);
   return launch_ok("attn_fwd_kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
 }
 
@@ -586,6 +583,12 @@ extern "C" int dtb_attn_launch_plan(const dtb_attn_params* p, int32_t sms, dtb_l
     out->slot[i] = live ? plan.table.slot[i] : -1;
   }
   return DTB_OK;
+}
+
+extern "C" int dtb_attn_block_rows(const dtb_attn_params* p, int32_t sms) {
+  if (check_params(p, false) != DTB_OK || sms < 0 || sms > 148) return 0;
+  if (p->num_splits != 0 && resolve_splits(p) > 1) return kQTiles * kBlockM;   // key splits have one form
+  return solo_blocks(p, sms == 0 ? current_sm_count() : sms) ? kBlockM : kQTiles * kBlockM;
 }
 
 extern "C" int dtb_attn_fwd(const dtb_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {

@@ -26,7 +26,7 @@ STATIC_SCRATCH_BYTES = 32 << 20
 # Every symbol the public header declares; tests check that the library exports all of them.
 EXPORTED_SYMBOLS = (
     "dtb_version", "dtb_status_string", "dtb_last_error_detail", "dtb_attn_supported", "dtb_attn_workspace_bytes",
-    "dtb_attn_fwd", "dtb_attn_launch_plan", "dtb_attn_fwd_static_scratch", "dtb_attn_fwd_scatter", "dtb_attn_fwd_sparse", "dtb_scatter_heads",
+    "dtb_attn_fwd", "dtb_attn_launch_plan", "dtb_attn_block_rows", "dtb_attn_fwd_static_scratch", "dtb_attn_fwd_scatter", "dtb_attn_fwd_sparse", "dtb_scatter_heads",
     "dtb_attn_fwd_residual", "dtb_attn_finalize", "dtb_fixed_m_operands", "dtb_qk_prepass", "dtb_quantize_e4m3",
     "dtb_smooth_k", "dtb_smooth_k_scratch_bytes", "dtb_fixed_m_from_norms", "dtb_out_proj", "dtb_sum_partials",
     "dtb_selftest_tmem_roundtrip", "dtb_selftest_qk", "dtb_selftest_pv", "dtb_selftest_wait_timeout",
@@ -179,6 +179,8 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
         lib.dtb_attn_fwd.argtypes = [ctypes.POINTER(AttnParams), vp, ctypes.c_size_t, vp]
         lib.dtb_attn_launch_plan.restype = ctypes.c_int
         lib.dtb_attn_launch_plan.argtypes = [ctypes.POINTER(AttnParams), ctypes.c_int32, ctypes.POINTER(LaunchPlan)]
+        lib.dtb_attn_block_rows.restype = ctypes.c_int
+        lib.dtb_attn_block_rows.argtypes = [ctypes.POINTER(AttnParams), ctypes.c_int32]
         lib.dtb_attn_fwd_static_scratch.restype = ctypes.c_int
         lib.dtb_attn_fwd_static_scratch.argtypes = [ctypes.POINTER(AttnParams), vp]
         lib.dtb_attn_fwd_sparse.restype = ctypes.c_int

@@ -327,11 +327,13 @@ def describe_launch(batch: int, heads: int, seq_q: int, seq_kv: Optional[int] = 
     p.q_stride_b = p.o_stride_b = heads * seq_q * 128
     p.k_stride_b = p.v_stride_b = heads * skv * 128
     plan = _lib.LaunchPlan()
-    _lib.check(_lib.load().dtb_attn_launch_plan(ctypes.byref(p), int(sms), ctypes.byref(plan)), "dtb_attn_launch_plan")
+    lib = _lib.load()
+    _lib.check(lib.dtb_attn_launch_plan(ctypes.byref(p), int(sms), ctypes.byref(plan)), "dtb_attn_launch_plan")
     n_sms = sms or 148
     head = f"{plan.units} query blocks x {plan.key_tiles} key tiles ({plan.units / n_sms:.2f} waves of {n_sms})"
     if plan.n_pieces == 0:
-        return head + ": plain launch, one CTA per query block"
+        rows = lib.dtb_attn_block_rows(ctypes.byref(p), int(sms))
+        return head + ": plain launch, one CTA per " + ("query block" if rows == 256 else f"{rows} rows of a query block")
     lens = [plan.tile_end[i] - plan.tile_begin[i] for i in range(plan.n_pieces)]
     return (head + f": {plan.whole_units} whole, the last {plan.tail_units} cut into {plan.n_pieces} pieces of "
             f"{min(lens)}-{max(lens)} key tiles ({plan.n_slots} merged through scratch)")

@@ -143,8 +143,8 @@ size_t dtb_attn_workspace_bytes(const dtb_attn_params* p);
  * units - numbered query block fastest, then head, then batch - are swept whole, one CTA each; when n_pieces > 0 the
  * remaining tail_units units are swept in n_pieces pieces, piece i being key tiles [tile_begin[i], tile_end[i]) of unit
  * unit[i], listed longest first; a piece with slot[i] >= 0 leaves its state in that scratch slot for the merge, and
- * the slots of one unit are consecutive in key order.  n_pieces == 0 means the plain launch, one CTA per unit or, where
- * that leaves SMs idle, one per 128-row half of a unit.  The plan depends only
+ * the slots of one unit are consecutive in key order.  n_pieces == 0 means the plain launch, whose CTAs take
+ * dtb_attn_block_rows rows each: one per unit, or one per 128-row half of a unit.  The plan depends only
  * on the static shape; it plays the role of the reference's per-shape tile resolution, which logs one line per
  * resolved shape (diffusers_tpu/kernels/mesh_attention.py:199-216, diffusers_tpu/kernels/block_sizes.py:442-577). */
 #define DTB_MAX_PIECES 304
@@ -157,6 +157,11 @@ typedef struct dtb_launch_plan {
 } dtb_launch_plan;
 
 int dtb_attn_launch_plan(const dtb_attn_params* p, int32_t sms, dtb_launch_plan* out);
+
+/* Query rows of one CTA, 256 or 128, in a launch without pieces (the plain launch of automatic and unsplit calls, and
+ * the residual, scatter, E4M3 and block-sparse forms) or with forced key splits; `sms` as above.  0: `p` or `sms` is not
+ * valid. */
+int dtb_attn_block_rows(const dtb_attn_params* p, int32_t sms);
 
 /* Normalised joint attention forward: o = softmax(scale * q k^T + key_mask) v.
  * Replaces diffusers_tpu/kernels/splash.py:566-650 `attention(...)` (and the per-sample loop around it

@@ -238,3 +238,22 @@ def test_describe_launch_names_the_form():
 
     assert "plain launch" in dtb200.describe_launch(2, 24, 4608)
     assert "cut into" in dtb200.describe_launch(1, 12, 4608)
+    assert dtb200.describe_launch(2, 24, 4608).endswith("one CTA per query block")
+    assert dtb200.describe_launch(2, 24, 333, 16731).endswith("one CTA per 128 rows of a query block")
+
+
+@pytest.mark.parametrize("B,H,Sq,Skv,rows", [(2, 24, 333, 16731, 128), (1, 3, 1280, 1280, 128), (1, 24, 1280, 1280, 256),
+                                             (2, 24, 4608, 4608, 256)])
+def test_block_rows_say_which_kernel_a_plain_launch_takes(B, H, Sq, Skv, rows):
+    lib = _lib.load()
+    p = _shape(B, H, Sq)
+    p.Skv = Skv
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), 148) == rows
+    p.num_splits = 1
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), 148) == rows
+    p.num_splits = 3
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), 148) == 256
+    p.num_splits = 0
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), 149) == 0
+    p.Hkv = 0
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), 148) == 0
