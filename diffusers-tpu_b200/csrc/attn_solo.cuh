@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     }
     if (ok && n_own > 0) ok = warp_wait(&bars->o_full[t], 0, ctx, SITE_O_FULL + t);
     // Group 1 hands over its (m, l); its O is read by group 0's warps, which see the same lanes.
-    float w_own = 1.f, w_other = 0.f;      // factors of O_0 and O_1
+    float w_own = 1.f, w_other = 1.f;      // factors of O_0 and O_1
     const bool merge = n_tiles > 1;
     if (merge && ok) {
       float2* ml = &bars->ml[row_in_tile];
@@ -361,10 +361,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
       } else {
         ok = warp_wait(&bars->solo_ready, 0, ctx, kSiteSoloReady) && warp_wait(&bars->o_full[1], 0, ctx, SITE_O_FULL + 1);
         if (ok) {
+          // A group whose sum is 0 has no say in the offset.  Any other sum has, NaN included, and both accumulators are
+          // always taken: what is not finite in either half of the keys shows in the output, as with one group.
           const float2 other = *ml;
-          const float m = other.y > 0.f && (other.x > m_used || !(l_sum > 0.f)) ? other.x : m_used;
-          if (l_sum > 0.f && m_used != m) w_own = ex2(m_used - m);
-          if (other.y > 0.f) w_other = other.x != m ? ex2(other.x - m) : 1.f;
+          const float m = other.y == 0.f ? m_used : l_sum == 0.f ? other.x : fmaxf(m_used, other.x);
+          w_own = l_sum == 0.f || m_used == m ? 1.f : ex2(m_used - m);
+          w_other = other.y == 0.f || other.x == m ? 1.f : ex2(other.x - m);
           l_sum = l_sum * w_own + other.y * w_other;
           m_used = m;
         }
@@ -379,10 +381,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
           uint32_t r1[32];
           tmem_ld32_sync(o_tmem + kBlockN + c * 32, r1);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float a = __uint_as_float(r[i]) * w_own;
-            r[i] = __float_as_uint(w_other > 0.f ? fmaf(__uint_as_float(r1[i]), w_other, a) : a);
-          }
+          for (int i = 0; i < 32; ++i)
+            r[i] = __float_as_uint(fmaf(__uint_as_float(r1[i]), w_other, __uint_as_float(r[i]) * w_own));
         }
       };
       if (kResidual) {

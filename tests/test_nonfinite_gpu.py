@@ -1,0 +1,62 @@
+"""NaN and infinity in the inputs come out as they do from float32 attention, whichever kernel and key tile meets them."""
+import ctypes
+
+import pytest
+import torch
+
+import dtb200
+from dtb200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda")
+SQ, SKV = 300, 1280                      # ten key tiles
+KERNELS = [(2, 128), (60, 256)]          # heads, rows of a CTA that this many heads lead to
+
+
+def _inputs(H, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    q, k, v = (torch.randn(1, H, s, 128, generator=g, device=DEV) for s in (SQ, SKV, SKV))
+    q, k = (t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True)) for t in (q, k))
+    return tuple(t.to(torch.bfloat16) for t in (q, k, v))
+
+
+def _reference(q, k, v):
+    return torch.softmax(q.float() @ k.float().transpose(-1, -2) * 128 ** -0.5, -1) @ v.float()
+
+
+def _run(kind, q, k, v, rows):
+    p = ops._fill_params(q, k, v, None, None, None, None, 0, 1, None)
+    assert _lib.load().dtb_attn_block_rows(ctypes.byref(p), 0) == rows
+    if kind == "plain":
+        out = dtb200.attention(q, k, v, num_splits=1)
+    else:                                # a second ring step meets the keys; the first one holds a copy of the first key tile
+        state = dtb200.ResidualState(1, q.shape[1], SQ, DEV)
+        dtb200.residual_attention_(state, q, k[:, :, :128], v[:, :, :128])
+        dtb200.residual_attention_(state, q, k, v, kv_offset=128)
+        out = state.o / state.l[..., None]
+    dtb200.check_device_status(DEV)
+    return out.float()
+
+
+def _check(out, ref):
+    assert torch.equal(out.isnan(), ref.isnan())
+    # bf16 probabilities and outputs, as in the other parity tests
+    assert (out - ref).nan_to_num(0.0).abs().max().item() <= 2e-2
+
+
+@pytest.mark.parametrize("H,rows", KERNELS)
+@pytest.mark.parametrize("kind", ["plain", "ring"])
+@pytest.mark.parametrize("what", ["nan", "inf", "value"])
+@pytest.mark.parametrize("key", [5, 130, 270, 1100, 1279])     # key tiles 0, 1, 2, 8 and 9
+def test_not_a_number_reaches_the_output(H, rows, kind, what, key):
+    q, k, v = _inputs(H, key)
+    if what == "nan":                    # every row of head 0 is NaN, no other head is
+        k[0, 0, key] = float("nan")
+    elif what == "value":                # one column of head 0 is NaN
+        v[0, 0, key, 7] = float("nan")
+    else:                                # logits of +inf for rows with q[0] > 0 (NaN), of -inf for the others (weight 0)
+        k[0, 0, key, 0] = 3e38
+        q[0, 0, :, 0] = torch.where(torch.arange(SQ, device=DEV) % 3 == 0, 2.0, -2.0).to(torch.bfloat16)
+    ref = _reference(q, k, v) if kind == "plain" else _reference(q, torch.cat([k[:, :, :128], k], 2), torch.cat([v[:, :, :128], v], 2))
+    assert ref.isnan().any()
+    _check(_run(kind, q, k, v, rows), ref)
