@@ -267,7 +267,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     const uint32_t bar_p_lo = smem_u32(&bars->p_lo[t]);
     const uint32_t bar_p_hi = smem_u32(&bars->p_hi[t]);
 
-    float m_used = -INFINITY;
+    // Group 1 starts from a finite offset.  Its first tile is not the first tile of the row: where all its logits are -inf,
+    // they weigh 0 beside those of tile 0, and -inf - (-inf) would make them NaN.
+    float m_used = t == 0 ? -INFINITY : kLowestOffset;
     float l_sum = 0.f;
     bool fixed_m = false;
     if (p.mk != nullptr && p.mk[p.Hq + h] > 0.5f) {

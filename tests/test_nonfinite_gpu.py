@@ -60,3 +60,17 @@ def test_not_a_number_reaches_the_output(H, rows, kind, what, key):
     ref = _reference(q, k, v) if kind == "plain" else _reference(q, torch.cat([k[:, :, :128], k], 2), torch.cat([v[:, :, :128], v], 2))
     assert ref.isnan().any()
     _check(_run(kind, q, k, v, rows), ref)
+
+
+@pytest.mark.parametrize("H,rows", KERNELS)
+@pytest.mark.parametrize("kind", ["plain", "ring"])
+@pytest.mark.parametrize("tiles", [(1,), (1, 2), (2, 3), (1, 3, 5, 7, 9), (9,)])
+@pytest.mark.parametrize("every", [1, 3])
+def test_key_tiles_whose_logits_are_all_minus_infinity_weigh_nothing(H, rows, kind, tiles, every):
+    q, k, v = _inputs(H, tiles[-1])
+    q[..., 0] = torch.where(torch.arange(SQ, device=DEV) % every == 0, 2.0, 0.0).to(torch.bfloat16)   # the other rows see them
+    for t in tiles:
+        k[:, :, 128 * t:128 * t + 128, 0] = -3e38
+    ref = _reference(q, k, v) if kind == "plain" else _reference(q, torch.cat([k[:, :, :128], k], 2), torch.cat([v[:, :, :128], v], 2))
+    assert not ref.isnan().any()
+    _check(_run(kind, q, k, v, rows), ref)
