@@ -307,20 +307,36 @@ constexpr int kPieceOverheadTiles = DTB_PIECE_OVERHEAD_TILES;
 // Key-tile times that a block costs beyond its key tiles: launch, pipeline fill and drain, epilogue.
 constexpr int kBlockOverheadTiles = 5;
 
-// Time of a launch with one CTA per block of `rows` query rows, in key-tile times.  A block with one query tile passes
-// two key tiles in the time of one.
-long long plain_time(const dtb_attn_params* p, int sms, int rows) {
+// Key tiles of the longest walk of a query block, as far as the static shape says: a block-sparse call visits no more
+// than its table is wide.  (Less than four is taken as four, from where a single round goes to 128-row blocks: it is
+// faster there at two tiles already, 74 / 148 blocks 10.6 / 9.4 us.)
+int key_tiles(const dtb_attn_params* p, const dtb_block_table* tb) {
+  const int n = (p->Skv + kBlockN - 1) / kBlockN;
+  return tb != nullptr ? std::min(n, std::max(tb->width, 4)) : n;
+}
+
+// Time of a launch with one CTA per block of `rows` query rows and n key tiles, in key-tile times.  A block with one
+// query tile passes two key tiles in the time of one.
+long long plain_time(const dtb_attn_params* p, int sms, int rows, long long n) {
   const long long blocks = static_cast<long long>((p->Sq + rows - 1) / rows) * p->Hq * p->B;
-  const long long n = (p->Skv + kBlockN - 1) / kBlockN;
   return (blocks + sms - 1) / sms * ((rows == kBlockM ? (n + 1) / 2 : n) + kBlockOverheadTiles);
 }
 
 // Whether `time` is worse than a launch of 128-row blocks.  Those read K and V once per 128 rows instead of once per
-// 256, which is paid for out of the margin: 144 blocks of 128 rows x 131 tiles take 187 us, 2.6 us per period, where a
-// period of 256-row blocks takes 1.6 to 1.9 us.  (54 blocks of 256 rows x 18 tiles: 35.2 us; 108 of 128 rows: 24.6 us.)
-bool solo_beats(const dtb_attn_params* p, int sms, long long time) { return 5 * plain_time(p, sms, kBlockM) < 4 * time; }
+// 256, which is paid for out of the margin.  Measured, 256-row blocks against 128-row ones, device time:
+//   one round each: 54 / 108 blocks x 18 tiles 34.6 / 23.6 us; 72 / 144 x 36 60.8 / 39.6; 96 / 144 x 132 221 / 157
+//   two rounds against three: 198 / 396 x 132 441 / 423 us in a loop of seconds, under the power limit (a ring step
+//   with that many 455 / 428, with E4M3 scores 441 / 383); 216 / 432 x 36 123 / 117, a model ratio of 0.84, left out
+//   the same with few tiles, as under a narrow table: 222 / 444 x 6 34.0 / 38.1 us, x 12 53.4 / 55.0, x 24 90.0 / 88.0
+//   one against two: 108 / 216 x 36 61.8 / 74.9 us
+bool solo_beats(const dtb_attn_params* p, int sms, int n, long long time) {
+  return 5 * plain_time(p, sms, kBlockM, n) < 4 * time;
+}
 
-bool solo_blocks(const dtb_attn_params* p, int sms) { return solo_beats(p, sms, plain_time(p, sms, kQTiles * kBlockM)); }
+bool solo_blocks(const dtb_attn_params* p, const dtb_block_table* tb, int sms) {
+  const int n = key_tiles(p, tb);
+  return solo_beats(p, sms, n, plain_time(p, sms, kQTiles * kBlockM, n));
+}
 
 struct BalancedPlan {
   bool use = false;
@@ -343,8 +359,9 @@ void plan_balanced(const dtb_attn_params* p, int sms, BalancedPlan* plan) {
   if (runs <= tail) return;
   const long long run_len = (tiles + runs - 1) / runs;
   if (run_len + kPieceOverheadTiles > n) return;   // the plain launch is as fast or faster
-  // ... and so may be 128-row blocks, where there are few blocks
-  if (solo_beats(p, sms, units / sms * (n + kBlockOverheadTiles) + run_len + kPieceOverheadTiles)) return;
+  // ... and so may be 128-row blocks, where there are few blocks.  (The pieces' overhead is taken as all that they cost
+  // here, not as what they cost beyond a block's own start and finish: where the two are close, the pieces stay.)
+  if (solo_beats(p, sms, n, units / sms * (n + kBlockOverheadTiles) + run_len + kPieceOverheadTiles)) return;
   struct Piece { int x, tb, te; };
   Piece pieces[kMaxPieces];
   int np = 0;
@@ -487,8 +504,8 @@ int fill_kernel_params(const dtb_attn_params* p, AttnKernelParams* kp) {
 
 // One CTA per query block, with 256-row blocks or (solo_blocks) 128-row ones.
 template <bool kResidual, bool kQkFp8>
-int launch_plain(const dtb_attn_params* p, const AttnKernelParams& kp, cudaStream_t s) {
-  if (solo_blocks(p, current_sm_count())) {
+int launch_plain(const dtb_attn_params* p, const AttnKernelParams& kp, cudaStream_t s, const dtb_block_table* tb = nullptr) {
+  if (solo_blocks(p, tb, current_sm_count())) {
     attn_solo_kernel<kResidual, kQkFp8><<<dim3((p->Sq + kBlockM - 1) / kBlockM, p->Hq, p->B), dim3(kNumThreads), kSoloSmemBytes, s>>>(kp);
     return launch_ok("attn_solo_kernel launch") ? DTB_OK : DTB_ERR_LAUNCH;
   }
@@ -585,10 +602,10 @@ extern "C" int dtb_attn_launch_plan(const dtb_attn_params* p, int32_t sms, dtb_l
   return DTB_OK;
 }
 
-extern "C" int dtb_attn_block_rows(const dtb_attn_params* p, int32_t sms) {
-  if (check_params(p, false) != DTB_OK || sms < 0 || sms > 148) return 0;
-  if (p->num_splits != 0 && resolve_splits(p) > 1) return kQTiles * kBlockM;   // key splits have one form
-  return solo_blocks(p, sms == 0 ? current_sm_count() : sms) ? kBlockM : kQTiles * kBlockM;
+extern "C" int dtb_attn_block_rows(const dtb_attn_params* p, const dtb_block_table* tb, int32_t sms) {
+  if (check_params(p, false) != DTB_OK || sms < 0 || sms > 148 || (tb != nullptr && tb->width < 1)) return 0;
+  if (tb == nullptr && p->num_splits != 0 && resolve_splits(p) > 1) return kQTiles * kBlockM;   // key splits have one form
+  return solo_blocks(p, tb, sms == 0 ? current_sm_count() : sms) ? kBlockM : kQTiles * kBlockM;
 }
 
 extern "C" int dtb_attn_fwd(const dtb_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {
@@ -866,7 +883,7 @@ extern "C" int dtb_attn_fwd_sparse(const dtb_attn_params* p, const dtb_block_tab
   kp.head_class = tb->n_classes > 1 ? tb->head_class : nullptr;
   kp.table_qblocks = tb->q_blocks;
   kp.table_width = tb->width;
-  return launch_plain<false, false>(p, kp, static_cast<cudaStream_t>(stream));
+  return launch_plain<false, false>(p, kp, static_cast<cudaStream_t>(stream), tb);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -180,7 +180,7 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
         lib.dtb_attn_launch_plan.restype = ctypes.c_int
         lib.dtb_attn_launch_plan.argtypes = [ctypes.POINTER(AttnParams), ctypes.c_int32, ctypes.POINTER(LaunchPlan)]
         lib.dtb_attn_block_rows.restype = ctypes.c_int
-        lib.dtb_attn_block_rows.argtypes = [ctypes.POINTER(AttnParams), ctypes.c_int32]
+        lib.dtb_attn_block_rows.argtypes = [ctypes.POINTER(AttnParams), ctypes.POINTER(BlockTable), ctypes.c_int32]
         lib.dtb_attn_fwd_static_scratch.restype = ctypes.c_int
         lib.dtb_attn_fwd_static_scratch.argtypes = [ctypes.POINTER(AttnParams), vp]
         lib.dtb_attn_fwd_sparse.restype = ctypes.c_int

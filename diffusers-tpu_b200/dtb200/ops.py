@@ -332,7 +332,7 @@ def describe_launch(batch: int, heads: int, seq_q: int, seq_kv: Optional[int] = 
     n_sms = sms or 148
     head = f"{plan.units} query blocks x {plan.key_tiles} key tiles ({plan.units / n_sms:.2f} waves of {n_sms})"
     if plan.n_pieces == 0:
-        rows = lib.dtb_attn_block_rows(ctypes.byref(p), int(sms))
+        rows = lib.dtb_attn_block_rows(ctypes.byref(p), None, int(sms))
         return head + ": plain launch, one CTA per " + ("query block" if rows == 256 else f"{rows} rows of a query block")
     lens = [plan.tile_end[i] - plan.tile_begin[i] for i in range(plan.n_pieces)]
     return (head + f": {plan.whole_units} whole, the last {plan.tail_units} cut into {plan.n_pieces} pieces of "

@@ -159,9 +159,9 @@ typedef struct dtb_launch_plan {
 int dtb_attn_launch_plan(const dtb_attn_params* p, int32_t sms, dtb_launch_plan* out);
 
 /* Query rows of one CTA, 256 or 128, in a launch without pieces (the plain launch of automatic and unsplit calls, and
- * the residual, scatter, E4M3 and block-sparse forms) or with forced key splits; `sms` as above.  0: `p` or `sms` is not
- * valid. */
-int dtb_attn_block_rows(const dtb_attn_params* p, int32_t sms);
+ * the residual, scatter and E4M3 forms, and the block-sparse one with its table `tb`, else NULL) or with forced key
+ * splits; `sms` as above.  Of the table only the width is read.  0: an argument is not valid. */
+int dtb_attn_block_rows(const dtb_attn_params* p, const dtb_block_table* tb, int32_t sms);
 
 /* Normalised joint attention forward: o = softmax(scale * q k^T + key_mask) v.
  * Replaces diffusers_tpu/kernels/splash.py:566-650 `attention(...)` (and the per-sample loop around it

@@ -248,12 +248,25 @@ def test_block_rows_say_which_kernel_a_plain_launch_takes(B, H, Sq, Skv, rows):
     lib = _lib.load()
     p = _shape(B, H, Sq)
     p.Skv = Skv
-    assert lib.dtb_attn_block_rows(ctypes.byref(p), 148) == rows
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), None, 148) == rows
     p.num_splits = 1
-    assert lib.dtb_attn_block_rows(ctypes.byref(p), 148) == rows
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), None, 148) == rows
     p.num_splits = 3
-    assert lib.dtb_attn_block_rows(ctypes.byref(p), 148) == 256
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), None, 148) == 256
     p.num_splits = 0
-    assert lib.dtb_attn_block_rows(ctypes.byref(p), 149) == 0
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), None, 149) == 0
     p.Hkv = 0
-    assert lib.dtb_attn_block_rows(ctypes.byref(p), 148) == 0
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), None, 148) == 0
+
+
+@pytest.mark.parametrize("H,S,width,rows", [(3, 18944, 2, 256), (3, 18944, 12, 256), (3, 18944, 148, 128), (3, 18944, 200, 128),
+                                            (6, 9216, 6, 256), (6, 9216, 72, 128), (1, 4608, 6, 128), (1, 4608, 2, 128),
+                                            (2, 18944, 24, 256)])
+def test_block_rows_of_a_sparse_call_follow_its_table(H, S, width, rows):
+    """444 blocks of 128 rows need three rounds where 222 of 256 need two, and that pays over long walks only."""
+    lib = _lib.load()
+    tb = _lib.BlockTable(4096, 4096, None, 1, (S + 255) // 256, width)      # of the table only the width is read
+    p = _shape(1, H, S)
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), ctypes.byref(tb), 148) == rows
+    tb.width = 0
+    assert lib.dtb_attn_block_rows(ctypes.byref(p), ctypes.byref(tb), 148) == 0

@@ -26,7 +26,7 @@ def _reference(q, k, v):
 
 def _run(kind, q, k, v, rows):
     p = ops._fill_params(q, k, v, None, None, None, None, 0, 1, None)
-    assert _lib.load().dtb_attn_block_rows(ctypes.byref(p), 0) == rows
+    assert _lib.load().dtb_attn_block_rows(ctypes.byref(p), None, 0) == rows
     if kind == "plain":
         out = dtb200.attention(q, k, v, num_splits=1)
     else:                                # a second ring step meets the keys; the first one holds a copy of the first key tile
