@@ -267,9 +267,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     const uint32_t bar_p_lo = smem_u32(&bars->p_lo[t]);
     const uint32_t bar_p_hi = smem_u32(&bars->p_hi[t]);
 
-    // Group 1 starts from a finite offset.  Its first tile is not the first tile of the row: where all its logits are -inf,
-    // they weigh 0 beside those of tile 0, and -inf - (-inf) would make them NaN.
-    float m_used = t == 0 ? -INFINITY : kLowestOffset;
+    // A state, and group 1, start from a finite offset.  Group 1's first tile is not the first tile of the row: where all
+    // its logits are -inf, they weigh 0 beside those of tile 0, and -inf - (-inf) would make them NaN.
+    float m_used = kResidual || t == 1 ? kLowestOffset : -INFINITY;
     float l_sum = 0.f;
     bool fixed_m = false;
     if (p.mk != nullptr && p.mk[p.Hq + h] > 0.5f) {
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
           tmem_wait_st();
         }
       } else {
-        m_used = m_in;
+        m_used = fmaxf(m_in, kLowestOffset);   // -inf: no key yet
       }
       l_sum = l_in;
     }

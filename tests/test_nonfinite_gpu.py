@@ -38,6 +38,21 @@ def _run(kind, q, k, v, rows):
     return out.float()
 
 
+def _merged(kind, q, k, v, kv_len=None):
+    """Calls whose results are merged from partial states by a kernel of their own."""
+    if kind == "ring":
+        state = dtb200.ResidualState(*q.shape[:3], DEV)
+        dtb200.residual_attention_(state, q, k, v, kv_len=kv_len)
+        out = dtb200.finalize_residual(state, kv_len=kv_len)
+    elif kind == "splits":
+        out = dtb200.attention(q, k, v, kv_len=kv_len, num_splits=3)
+    else:
+        assert "cut into" in dtb200.describe_launch(*q.shape[:3], k.shape[2])
+        out = dtb200.attention(q, k, v, kv_len=kv_len)
+    dtb200.check_device_status(DEV)
+    return out.float()
+
+
 def _check(out, ref):
     assert torch.equal(out.isnan(), ref.isnan())
     # bf16 probabilities and outputs, as in the other parity tests
@@ -74,3 +89,18 @@ def test_key_tiles_whose_logits_are_all_minus_infinity_weigh_nothing(H, rows, ki
     ref = _reference(q, k, v) if kind == "plain" else _reference(q, torch.cat([k[:, :, :128], k], 2), torch.cat([v[:, :, :128], v], 2))
     assert not ref.isnan().any()
     _check(_run(kind, q, k, v, rows), ref)
+
+
+@pytest.mark.parametrize("kind,H,S,first", [("ring", 1, 300, 0), ("ring", 2, 1280, 0), ("ring", 60, 1280, 1), ("splits", 1, 1280, 0),
+                                            ("splits", 1, 1280, 1), ("pieces", 1, 4608, 0), ("pieces", 1, 4608, 1), ("pieces", 12, 4608, 1)])
+def test_partial_states_that_start_with_minus_infinity_keep_their_other_keys(kind, H, S, first):
+    """Every other key tile, from ``first`` on, is all -inf for two rows of three; some states begin with such a tile."""
+    g = torch.Generator(device=DEV).manual_seed(S + first)
+    q, k, v = (torch.randn(1, H, S, 128, generator=g, device=DEV) for _ in range(3))
+    q, k = (t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True)) for t in (q, k))
+    q[..., 0] = torch.where(torch.arange(S, device=DEV) % 3 == 0, 0.0, 2.0)
+    k[..., 0] = torch.where(torch.arange(S, device=DEV) // 128 % 2 == first, -3e38, 0.5)
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    out = _merged(kind, q, k, v)
+    for h in range(H):
+        _check(out[:, h], _reference(q[:, h], k[:, h], v[:, h]))
