@@ -21,7 +21,8 @@ constexpr int kNumSms = 148;
 
 // ---------------------------------------------------------------------------
 // Merge `num` partial states per row and write the normalised bf16 output.
-// One warp per query row; lane i owns output columns 4i..4i+3.
+// One warp per query row; lane i owns output columns 4i..4i+3.  A state is left out where its sum is 0, and only there:
+// a NaN sum is the row's result.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ acc_o, const float* __restrict__ acc_m,
                                                       const float* __restrict__ acc_l, int num, int B, int Hq, int Sq,
@@ -39,13 +40,13 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
   for (int i = 0; i < num; ++i) {
     const float l = acc_l[i * rows + rid];
     const float m = acc_m[i * rows + rid];
-    if (l > 0.f) m_max = fmaxf(m_max, m);
+    if (l != 0.f) m_max = fmaxf(m_max, m);
   }
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float l_tot = 0.f;
   for (int i = 0; i < num; ++i) {
     const float l = acc_l[i * rows + rid];
-    if (!(l > 0.f)) continue;
+    if (l == 0.f) continue;
     const float w = exp2f(acc_m[i * rows + rid] - m_max);
     l_tot += l * w;
     const float4 v = reinterpret_cast<const float4*>(acc_o + (i * rows + rid) * kHeadDim)[lane];
@@ -55,7 +56,8 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
     acc.w += v.w * w;
   }
   const bool padded = zero_padded_rows && kv_len != nullptr && (q_offset + s >= kv_len[b]);
-  const float inv = (l_tot > 0.f && !padded) ? 1.0f / l_tot : 0.f;
+  const float inv = l_tot > 0.f ? 1.0f / l_tot : 0.f;
+  if (padded) acc = make_float4(0.f, 0.f, 0.f, 0.f);
   uint2 packed;
   packed.x = pack_bf16x2(acc.x * inv, acc.y * inv);
   packed.y = pack_bf16x2(acc.z * inv, acc.w * inv);
@@ -114,7 +116,7 @@ __global__ void __launch_bounds__(256) merge_pieces_kernel(const __grid_constant
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (i0 + u < count && l4[u] > 0.f) m_max = fmaxf(m_max, m4[u]);
+      if (i0 + u < count && l4[u] != 0.f) m_max = fmaxf(m_max, m4[u]);
   }
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float l_tot = 0.f;
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(256) merge_pieces_kernel(const __grid_constant
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      if (i0 + u < count && l4[u] > 0.f) {     // a piece with no valid key wrote no o: never touch it
+      if (i0 + u < count && l4[u] != 0.f) {    // a piece with no valid key wrote no o: never touch it
         const float w = exp2f(m4[u] - m_max);
         l_tot += l4[u] * w;
         acc.x += v4[u].x * w;
@@ -141,7 +143,8 @@ __global__ void __launch_bounds__(256) merge_pieces_kernel(const __grid_constant
     }
   }
   const bool padded = zero_padded_rows && kv_len != nullptr && (s >= kv_len[b]);
-  const float inv = (l_tot > 0.f && !padded) ? 1.0f / l_tot : 0.f;
+  const float inv = l_tot > 0.f ? 1.0f / l_tot : 0.f;
+  if (padded) acc = make_float4(0.f, 0.f, 0.f, 0.f);
   uint2 packed;
   packed.x = pack_bf16x2(acc.x * inv, acc.y * inv);
   packed.y = pack_bf16x2(acc.z * inv, acc.w * inv);

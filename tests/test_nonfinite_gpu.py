@@ -104,3 +104,25 @@ def test_partial_states_that_start_with_minus_infinity_keep_their_other_keys(kin
     out = _merged(kind, q, k, v)
     for h in range(H):
         _check(out[:, h], _reference(q[:, h], k[:, h], v[:, h]))
+
+
+@pytest.mark.parametrize("kind,S", [("ring", 500), ("splits", 1280), ("pieces", 4608)])
+@pytest.mark.parametrize("tile", [0, 1, 2, 3])
+def test_not_a_number_passes_through_a_merge(kind, S, tile):
+    g = torch.Generator(device=DEV).manual_seed(tile)
+    q, k, v = (torch.randn(1, 1, S, 128, generator=g, device=DEV).to(torch.bfloat16) for _ in range(3))
+    k[0, 0, 128 * tile + 9, 0] = 3e38                       # +inf or -inf, by the sign of q
+    q[..., 0] = torch.where(torch.arange(S, device=DEV) % 3 == 0, 2.0, -2.0).to(torch.bfloat16)
+    ref = _reference(q, k, v)
+    assert ref.isnan().any() and not ref.isnan().all()
+    out = _merged(kind, q, k, v)
+    assert torch.equal(out.isnan(), ref.isnan())
+
+
+@pytest.mark.parametrize("kind,S", [("ring", 500), ("splits", 1280), ("pieces", 4608)])
+def test_a_merge_zeroes_padded_queries_whatever_they_hold(kind, S):
+    g = torch.Generator(device=DEV).manual_seed(S)
+    q, k, v = (torch.randn(1, 1, S, 128, generator=g, device=DEV).to(torch.bfloat16) for _ in range(3))
+    q[:, :, S - 70:] = float("nan")
+    out = _merged(kind, q, k, v, kv_len=[S - 70])
+    assert out[:, :, S - 70:].abs().max().item() == 0.0 and not out.isnan().any()
