@@ -83,11 +83,12 @@ def test_eight_gpu_drivers(mode, shape):
     _run_ranks(8, mode, *shape)
 
 
-@pytest.mark.parametrize("P,B,H,Sl,balanced", [
-    (4, 2, 8, 160, False),
-    (2, 1, 24, 2304, True),      # 216 units per rank: the automatic call balances its last wave and merges to the peers
+@pytest.mark.parametrize("P,B,H,Sl,balanced,rows", [
+    (4, 2, 8, 160, False, 256),
+    (4, 2, 8, 256, False, 128),  # few long blocks: 128-row ones
+    (2, 1, 24, 2304, True, 256), # 216 units per rank: the automatic call balances its last wave and merges to the peers
 ])
-def test_scatter_entry_points_with_local_buffers_as_peers(P, B, H, Sl, balanced):
+def test_scatter_entry_points_with_local_buffers_as_peers(P, B, H, Sl, balanced, rows):
     """One GPU stands in for the ranks: the `peer` buffers are ordinary local tensors."""
     import ctypes
 
@@ -120,6 +121,7 @@ def test_scatter_entry_points_with_local_buffers_as_peers(P, B, H, Sl, balanced)
     for rank in range(P):
         p = ops._fill_params(y[0][rank], y[1][rank], y[2][rank], None, kv_len, None, None, _lib.FLAG_ZERO_PADDED_ROWS,
                              0 if balanced else 1, ops._status_buffer(dev))
+        assert lib.dtb_attn_block_rows(ctypes.byref(p), None, 0) == rows
         sc = _lib.AttnScatter()
         if balanced:
             need = lib.dtb_attn_workspace_bytes(ctypes.byref(p))
