@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(256) merge_pieces_kernel(const __grid_constant
 // Max L2 row norm per head of a bf16 [B,H,S,128] tensor, folded into norms[h] with an integer atomic max (norms are
 // non-negative).  One block per (chunk of rows, head, batch element); a warp reads a whole 256-byte row per load,
 // eight rows in flight, and the block ends in one atomic.  HBM-bound: the tensor is read once.  (Rows dealt to warps
-// over the whole tensor, each warp at another head with every row and so at a global atomic per row, took 130 us per
-// 113 MB tensor; a bounded-logit call on 2 x 24 x 4608 rows went from 708 to 487 us with this split.)
+// over the whole tensor, each warp at another head with every row and so at a global atomic per row: q and k of 2 x 24 x
+// 4608 rows, 57 MB each, took 294 us a call, 39.5 with this split.)
 // ---------------------------------------------------------------------------
 constexpr int kNormRows = 256;         // rows of a block
 constexpr int kNormRowsInFlight = 8;   // per warp
@@ -892,9 +892,9 @@ extern "C" int dtb_attn_fwd_sparse(const dtb_attn_params* p, const dtb_block_tab
 // ---------------------------------------------------------------------------------------------
 // Saturating E4M3 cast of a bf16 [B, H, S, 128] tensor (values are multiplied by `mult` first, beyond +-448 they
 // clamp instead of overflowing), written contiguously.  One block per 128 rows of a head, 16 lanes per row, eight
-// 16-byte loads in flight per thread.  HBM-bound: 256 bytes in and 128 out per row.  (A
-// grid-stride loop over 16-byte chunks, with three 64-bit divisions for each, cost a call on 2 x 24 x 16896 rows 50 us
-// more: 5365 -> 5315 us with the score product in 8 bits.)
+// 16-byte loads in flight per thread.  HBM-bound: 256 bytes in and 128 out per row.  (A grid-stride loop over 16-byte
+// chunks, with three 64-bit divisions for each: 2 x 24 x 16896 rows, 311 MB, took 74.3 us, 48.7 so; 2 x 24 x 4608, launch
+// included, 23.1 and 16.4.)
 // ---------------------------------------------------------------------------------------------
 namespace dtb {
 namespace {
