@@ -4,28 +4,34 @@
 // Warp roles (384 threads = 3 warpgroups):
 //   warps 0-3   softmax group 0: one thread per query row of tile 0
 //   warps 4-7   softmax group 1: one thread per query row of tile 1
-//   warp  8     MMA issuer (one elected lane issues tcgen05.mma; the warp stays converged)
+//   warp  8     issuer of Q K^T (one elected lane issues tcgen05.mma; the warp stays converged)
 //   warp  9     TMA producer (lane 0 issues the tensor loads)
-//   warps 10-11 idle; they exist so that warps 8-11 form a whole warpgroup, which is the
+//   warp  10    issuer of P V
+//   warp  11    idle; it exists so that warps 8-11 form a whole warpgroup, which is the
 //               unit setmaxnreg works on: that warpgroup hands registers to the softmax groups
 //               (each SM sub-partition holds 16384 registers shared by one warp of each group).
 //
-// Tensor memory (512 columns): S0 | S1 | O0 | O1, 128 f32 columns each.  P (bf16)
-// is written over the first 64 columns of its S tile (in two halves, each with its
-// own mbarrier) and consumed from tensor memory by the PV MMA, so probabilities never
-// touch shared memory.
+// Tensor memory (512 columns): S | P0 | P1 | O0 | O1 - one S of 128 f32 columns that the two groups use in turn,
+// a P (128 keys in bf16, 64 columns) and an O (128 f32 columns) for each.  A group reads its S row into registers in one
+// load and gives S back at once, so the next Q K^T waits for that load of the other group and not, as it would with P
+// written over S, for this group's softmax and P V.  P is written in two halves, each with its own mbarrier, and
+// consumed from tensor memory by the P V MMA, so probabilities never touch shared memory.
 //
 // Shared memory: Q (2 x 32 KB, loaded once) and a ring of 32 KB slots through
-// which K_0, V_0, K_1, V_1, ... flow; every tile is two 64-column panels written
+// which K_0, K_1, V_0, K_2, V_1, ... flow; every tile is two 64-column panels written
 // by TMA with the 128-byte swizzle the MMA descriptors expect.
 //
-// The two softmax groups ping-pong: while group 0 exponentiates S0 the tensor
-// core runs P1*V and the next Q1*K^T, and vice versa.  MMAs issued by one thread
-// execute in order, which is what makes the S/P aliasing and the O rescale safe:
-//   * S_t(j+1) = Q_t K_{j+1}^T is issued after O_t += P_t(j) V_j, so it cannot
-//     overwrite P_t(j) early;
-//   * the commit that publishes S_t(j) follows PV_t(j-1) in issue order, so a
-//     softmax thread that has seen S_t(j) may read-modify-write O_t.
+// Order between the warps, all of it by mbarriers (t is the query tile, j the key tile):
+//   * Q_t K_j^T may overwrite S once the other group has arrived on s_free for the S before it;
+//   * group t writes P_t(j), or rescales O_t, once pv_done says that P_t(j-1) V_{j-1} has run;
+//   * P_t(j) V_j is issued after the group's arrivals on p_lo and p_hi.
+// Q K^T and P V touch disjoint columns, so the two issuers need no order between them.  They are two warps because a
+// warp does not get past a group of MMAs before the tensor pipe has taken them up: with both kinds in one warp, each wait
+// between two groups is idle time of the pipe (2 x 24 x 16896 rows: 5100 us, 4965 with two warps).
+//
+// What bounds it: the chain S -> registers -> next Q K^T -> S, twice per key tile, and the MUFU unit's 2048 cycles of
+// exponentials per key tile beside 2048 of tensor pipe.  Measured per call with P over S and one issuer / so, 2 x 24
+// heads: 16896 rows 4888 / 4710 us, 4608 rows 387 / 371, E4M3 scores 4850 / 4550.
 #pragma once
 
 #include "ptx.cuh"
@@ -40,8 +46,9 @@ constexpr int kStages = 4;                   // K/V ring slots
 constexpr uint32_t kPanelBytes = 128 * 64 * 2;
 constexpr uint32_t kTileBytes = 2 * kPanelBytes;
 constexpr int kNumSoftmaxThreads = kQTiles * kBlockM;
-constexpr int kMmaWarp = kNumSoftmaxThreads / 32;
+constexpr int kMmaWarp = kNumSoftmaxThreads / 32;   // issues Q K^T
 constexpr int kLoadWarp = kMmaWarp + 1;
+constexpr int kPvWarp = kMmaWarp + 2;               // issues P V
 constexpr int kNumThreads = kNumSoftmaxThreads + 128;
 // Register hand-over between warpgroups.  The kernel is compiled for kLaunchRegs registers per thread (what
 // 384 threads can have at most, rounded down to a multiple of 8; the host side refuses to launch a build
@@ -64,10 +71,11 @@ struct __align__(8) PipelineBarriers {
   uint64_t q_full[kQTiles];
   uint64_t kv_full[kStages];
   uint64_t kv_empty[kStages];
-  uint64_t s_full[kQTiles];
+  uint64_t s_full[kQTiles];    // S holds Q_t K_j^T
   uint64_t p_lo[kQTiles];   // first 64 keys of P_t written
   uint64_t p_hi[kQTiles];   // last 64 keys of P_t written
-  uint64_t o_full[kQTiles];
+  uint64_t pv_done[kQTiles];   // P_t V of a tile has run: P_t may be written again, O_t is whole
+  uint64_t s_free;          // S has been read into registers (by the two groups in turn)
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -77,7 +85,7 @@ constexpr size_t kSmemBytes = 1024 /* alignment slack */ + kQTiles * kTileBytes 
 
 // Barrier-site ids reported in status[1] when a wait runs out.
 enum WaitSite : int {
-  SITE_Q_FULL = 10, SITE_KV_FULL = 20, SITE_KV_EMPTY = 30, SITE_S_FULL = 40, SITE_P_FULL = 50, SITE_P_HI = 55, SITE_O_FULL = 60
+  SITE_Q_FULL = 10, SITE_KV_FULL = 20, SITE_KV_EMPTY = 30, SITE_S_FULL = 40, SITE_P_FULL = 50, SITE_P_HI = 55, SITE_O_FULL = 60, SITE_S_FREE = 65
 };
 
 struct AttnKernelParams {
@@ -136,18 +144,22 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const 
 // ---------------------------------------------------------------------------
 // One key tile of softmax for the row owned by this thread.
 //
-// The whole S row comes out of tensor memory in one load; the row max uses three-input max; the
-// scale-and-subtract and the row sum run on packed f32 pairs; P goes back to tensor memory in two
-// halves of 64 keys, each published on its own mbarrier so the PV MMA of the first half runs while
-// the second half is still being exponentiated.  Once the rows have an offset, the first half is exponentiated
-// with it before the row max is known (see below): the max then only confirms that the offset can stay.
+// The whole S row comes out of tensor memory in one load, after which S belongs to the other group; the row max uses
+// three-input max; the scale-and-subtract and the row sum run on packed f32 pairs; P goes to tensor memory in two halves
+// of 64 keys, each published on its own mbarrier so the PV MMA of the first half runs while the second half is still
+// being exponentiated.  wait_pv() returns when the P V of the group's tile before has run; with online softmax it stands in front
+// of the exponentials so that the first 32 probabilities can be stored under them (behind them: 371 -> 393 us on the
+// 1024-pixel shape).  Returns false when a wait ran out.  Exponentiating the first half before the maximum is known, which paid
+// while the next Q K^T waited for P, costs 6% now (371 -> 394 us).
 // ---------------------------------------------------------------------------
-template <bool kFixedM>
-__device__ __forceinline__ void softmax_tile(uint32_t s_tmem, uint32_t o_tmem, float scale_log2, int valid_cols,
-                                             bool o_live, float& m_used, float& l_sum, uint32_t bar_p_lo,
-                                             uint32_t bar_p_hi) {
+template <bool kFixedM, class WaitPv>
+__device__ __forceinline__ bool softmax_tile(uint32_t s_tmem, uint32_t p_tmem, uint32_t o_tmem, float scale_log2, int valid_cols,
+                                             bool o_live, float& m_used, float& l_sum, uint32_t bar_s_free, uint32_t bar_p_lo,
+                                             uint32_t bar_p_hi, WaitPv wait_pv) {
   uint32_t sr[kBlockN];
   tmem_ld128_sync(s_tmem, sr);
+  tc_fence_before();
+  mbar_arrive(bar_s_free);
   if (valid_cols < kBlockN) {
 #pragma unroll
     for (int i = 0; i < kBlockN; ++i)
@@ -157,8 +169,8 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_tmem, uint32_t o_tmem, f
   uint64_t acc2 = pack_f32x2(0.f, 0.f);
   uint32_t pk[32];
   // 2^(s * scale - m) for 64 keys: packed into pk, summed into acc2.
-  auto exp_half = [&](int half, float m) {
-    const uint64_t neg_m2 = pack_f32x2(-m, -m);
+  auto exp_half = [&](int half, bool store_first) {
+    const uint64_t neg_m2 = pack_f32x2(-m_used, -m_used);
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       const int col = half * 64 + 2 * i;
@@ -170,21 +182,16 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_tmem, uint32_t o_tmem, f
       acc2 = add_f32x2(acc2, pack_f32x2(p0, p1));
       pk[i] = pack_bf16x2(p0, p1);
       // The first 32 keys of the half go to tensor memory while the other 32 are exponentiated, which hides half
-      // of the store's latency.  Nothing reads them before the arrive in publish(), so a speculated half that is
-      // thrown away is simply overwritten.
-      if (i == 15) tmem_st16(s_tmem + half * 32, pk);
+      // of the store's latency.  Nothing reads them before the arrive in publish().
+      if (store_first && i == 15) tmem_st16(p_tmem + half * 32, pk);
     }
   };
-  auto publish = [&](int half) {
-    tmem_st16(s_tmem + half * 32 + 16, pk + 16);
+  auto publish = [&](int half, bool first_stored) {
+    if (!first_stored) tmem_st16(p_tmem + half * 32, pk);
+    tmem_st16(p_tmem + half * 32 + 16, pk + 16);
     tmem_wait_st();
     tc_fence_before();
     mbar_arrive(half == 0 ? bar_p_lo : bar_p_hi);
-  };
-  auto finish = [&]() {
-    float a0, a1;
-    unpack_f32x2(acc2, a0, a1);
-    l_sum += a0 + a1;
   };
   // The row maximum in log2 units: eight independent chains of three-input max keep the dependency depth at 8 + 3.
   auto row_max = [&]() {
@@ -200,26 +207,9 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_tmem, uint32_t o_tmem, f
   };
 
   if (!kFixedM) {
-    // The maximum only decides whether the offset in use has to move, which after the first tiles is rare
-    // (kRescaleThreshold).  So once every row of the warp has an offset, the first half of P is exponentiated with
-    // it in the same straight-line code as the reduction of the maximum - the exponentials wait on the MUFU unit,
-    // the maxima fill the issue slots between them - and that work is thrown away only if some row does move.
-    // On the 1024-pixel image shape this takes a call from 398 to 390 us.
-    if (__all_sync(0xffffffffu, m_used > kLowestOffset)) {
-      exp_half(0, m_used);
-      const float mx = row_max();
-      if (!__any_sync(0xffffffffu, mx > m_used + kRescaleThreshold)) {
-        publish(0);
-        exp_half(1, m_used);
-        publish(1);
-        finish();
-        return;
-      }
-      acc2 = pack_f32x2(0.f, 0.f);
-      tmem_wait_st();   // the speculated store has to land before the same columns are written again
-    }
     const float mx = row_max();
     const bool grow = mx > m_used + kRescaleThreshold;  // always true while m_used is -inf or kLowestOffset, for finite logits
+    if (!wait_pv()) return false;
     if (o_live && __any_sync(0xffffffffu, grow)) {
       const float alpha = grow ? ex2(m_used - mx) : 1.0f;
       l_sum *= alpha;
@@ -237,12 +227,19 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_tmem, uint32_t o_tmem, f
       l_sum *= ex2(m_used - mx);
     }
     if (grow) m_used = mx;
+    exp_half(0, true);
+    publish(0, true);
+  } else {
+    exp_half(0, false);
+    if (!wait_pv()) return false;
+    publish(0, false);
   }
-  exp_half(0, m_used);
-  publish(0);
-  exp_half(1, m_used);
-  publish(1);
-  finish();
+  exp_half(1, true);
+  publish(1, true);
+  float a0, a1;
+  unpack_f32x2(acc2, a0, a1);
+  l_sum += a0 + a1;
+  return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -361,8 +358,9 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
       mbar_init(smem_u32(&bars->s_full[i]), 1);
       mbar_init(smem_u32(&bars->p_lo[i]), kBlockM);
       mbar_init(smem_u32(&bars->p_hi[i]), kBlockM);
-      mbar_init(smem_u32(&bars->o_full[i]), 1);
+      mbar_init(smem_u32(&bars->pv_done[i]), 1);
     }
+    mbar_init(smem_u32(&bars->s_free), kBlockM);
     for (int i = 0; i < kStages; ++i) {
       mbar_init(smem_u32(&bars->kv_full[i]), 1);
       mbar_init(smem_u32(&bars->kv_empty[i]), 1);
@@ -383,6 +381,10 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
+  // Places in the K/V ring, in the order in which the issuer takes the tiles: K_0 K_1 V_0 K_2 V_1 ... K_{n-1} V_{n-2} V_{n-1}.
+  auto place_k = [&](int e) { return e == 0 ? 0 : 2 * e - 1; };
+  auto place_v = [&](int e) { return e == n_tiles - 1 ? 2 * n_tiles - 1 : 2 * e + 2; };
+
   if (warp == kLoadWarp) {
     // ------------------------------------------------------------------ TMA producer
     setmaxnreg_dec<kRegsService>();
@@ -401,10 +403,11 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
         if (use > 0) ok = mbar_wait(smem_u32(&bars->kv_empty[slot]), (use - 1) & 1, ctx, SITE_KV_EMPTY + slot);
         if (!ok) break;
         const uint32_t bar = smem_u32(&bars->kv_full[slot]);
-        const bool is_v = (i & 1) != 0;
+        const bool last = i == 2 * n_tiles - 1;
+        const bool is_v = last || (i > 0 && (i & 1) == 0);
         mbar_expect_tx(bar, is_v ? kTileBytes : kQkTileBytes);
         const uint32_t dst = smem_u32(smem_kv + slot * kTileBytes);
-        const int entry = tile_begin + (i >> 1);
+        const int entry = tile_begin + (last ? n_tiles - 1 : is_v ? (i - 2) >> 1 : (i + 1) >> 1);
         const int row = (tile_list != nullptr ? tile_list[entry] : entry) * kBlockN;
         const CUtensorMap* tm = is_v ? &p.tmap_v : &p.tmap_k;
         tma_load_4d(dst, tm, bar, 0, row, hk, b);
@@ -413,13 +416,11 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
     }
     __syncwarp();
   } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------------ issuer of S_t(j) = Q_t K_j^T
     setmaxnreg_dec<kRegsService>();
     constexpr uint32_t idesc_qk = kQkFp8 ? make_idesc_e4m3(kBlockM, kBlockN) : make_idesc_bf16(kBlockM, kBlockN, false, false);
-    constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, kHeadDim, false, true);
     const uint64_t q_desc0 = make_smem_desc_sw128(smem_u32(smem_q), 16, 1024);
     const uint64_t k_desc0 = make_smem_desc_sw128(smem_u32(smem_kv), 16, 1024);
-    const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(smem_kv), kPanelBytes, 1024);
     bool ok = true;
 
     // The issuing regions are entered through elect.sync rather than `lane == 0`: with the same instructions inside,
@@ -433,24 +434,47 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
 #pragma unroll
           for (int kk = 0; kk < kHeadDim / 32; ++kk) {   // 32 one-byte elements = 32 bytes of the swizzled row
             const uint64_t off = static_cast<uint64_t>((kk * 32) >> 4);
-            mma_ss_f8(tmem_base + t * kBlockN, a0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
+            mma_ss_f8(tmem_base, a0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
         } else {
 #pragma unroll
           for (int kk = 0; kk < kHeadDim / 16; ++kk) {
             const uint64_t off = static_cast<uint64_t>(((kk & 3) * 32 + (kk >> 2) * kPanelBytes) >> 4);
-            mma_ss(tmem_base + t * kBlockN, a0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
+            mma_ss(tmem_base, a0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
         }
         mma_commit(smem_u32(&bars->s_full[t]));
       }
       __syncwarp();
     };
+    auto commit_to = [&](uint64_t* bar) {
+      if (elect_one()) mma_commit(smem_u32(bar));
+      __syncwarp();
+    };
+
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const int i = place_k(j), slot = i % kStages;
+      for (int t = 0; t < kQTiles && ok; ++t) {
+        if (j == 0) ok = warp_wait(&bars->q_full[t], 0, ctx, SITE_Q_FULL + t);
+        if (ok && t == 0) ok = warp_wait(&bars->kv_full[slot], (i / kStages) & 1, ctx, SITE_KV_FULL + slot);
+        if (ok && (j > 0 || t > 0)) ok = warp_wait(&bars->s_free, (t + 1) & 1, ctx, SITE_S_FREE);
+        if (!ok) break;
+        tc_fence_after();
+        issue_qk(t, slot);
+        if (t == kQTiles - 1) commit_to(&bars->kv_empty[slot]);
+      }
+    }
+  } else if (warp == kPvWarp) {
+    // ------------------------------------------------------------------ issuer of O_t += P_t(j) V_j
+    setmaxnreg_dec<kRegsService>();
+    constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, kHeadDim, false, true);
+    const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(smem_kv), kPanelBytes, 1024);
+    bool ok = true;
     auto issue_pv = [&](int t, int slot, int half, bool accumulate) {
       if (elect_one()) {
         const uint64_t b0 = v_desc0 + static_cast<uint64_t>((slot * kTileBytes) >> 4);
         const uint32_t d_tmem = tmem_base + (kQTiles + t) * kBlockN;
-        const uint32_t a_tmem = tmem_base + t * kBlockN;
+        const uint32_t a_tmem = tmem_base + kBlockN + t * (kBlockN / 2);
 #pragma unroll
         for (int kk = half * 4; kk < half * 4 + 4; ++kk) {
           const uint64_t off = static_cast<uint64_t>((kk * 16 * 128) >> 4);
@@ -463,46 +487,21 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
       if (elect_one()) mma_commit(smem_u32(bar));
       __syncwarp();
     };
-    auto wait_kv = [&](int i) {
-      const int slot = i % kStages;
-      return warp_wait(&bars->kv_full[slot], (i / kStages) & 1, ctx, SITE_KV_FULL + slot);
-    };
-
-    // Prologue: S_t(0) = Q_t K_0^T for both tiles.
-    ok = warp_wait(&bars->q_full[0], 0, ctx, SITE_Q_FULL);
-    if (ok) ok = wait_kv(0);
-    if (ok) {
-      tc_fence_after();
-      issue_qk(0, 0);
-      ok = warp_wait(&bars->q_full[1], 0, ctx, SITE_Q_FULL + 1);
-    }
-    if (ok) {
-      tc_fence_after();
-      issue_qk(1, 0);
-      commit_to(&bars->kv_empty[0]);
-    }
     const bool o_preloaded = kResidual && !p.acc_init;
     for (int j = 0; j < n_tiles && ok; ++j) {
-      const int iv = 2 * j + 1;
-      const int ik = 2 * j + 2;
-      // No wait for V_j or K_{j+1} here: softmax group 0 checks both loads before it publishes P_0(j) (see
-      // there), so the P barriers below already say that the tiles have landed.
+      const int i = place_v(j), slot = i % kStages;
       for (int t = 0; t < kQTiles && ok; ++t) {
-        ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);
+        if (t == 0) ok = warp_wait(&bars->kv_full[slot], (i / kStages) & 1, ctx, SITE_KV_FULL + slot);
+        if (ok) ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);
         if (!ok) break;
         tc_fence_after();
-        issue_pv(t, iv % kStages, 0, j > 0 || o_preloaded);
+        issue_pv(t, slot, 0, j > 0 || o_preloaded);
         ok = warp_wait(&bars->p_hi[t], j & 1, ctx, SITE_P_HI + t);
         if (!ok) break;
         tc_fence_after();
-        issue_pv(t, iv % kStages, 1, true);
-        if (t == kQTiles - 1) commit_to(&bars->kv_empty[iv % kStages]);
-        if (j + 1 < n_tiles) {
-          issue_qk(t, ik % kStages);
-          if (t == kQTiles - 1) commit_to(&bars->kv_empty[ik % kStages]);
-        } else {
-          commit_to(&bars->o_full[t]);
-        }
+        issue_pv(t, slot, 1, true);
+        commit_to(&bars->pv_done[t]);
+        if (t == kQTiles - 1) commit_to(&bars->kv_empty[slot]);
       }
     }
   } else if (warp < kMmaWarp) {
@@ -512,11 +511,13 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
     const int row_in_tile = threadIdx.x & (kBlockM - 1);
     const int row = q0 + t * kBlockM + row_in_tile;  // query row within this call
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_tmem = tmem_base + lane_off + t * kBlockN;
+    const uint32_t s_tmem = tmem_base + lane_off;
+    const uint32_t p_tmem = tmem_base + lane_off + kBlockN + t * (kBlockN / 2);
     const uint32_t o_tmem = tmem_base + lane_off + (kQTiles + t) * kBlockN;
     const float scale_log2 = p.scale_log2;
     const bool row_in_range = row < p.Sq;
     const int64_t acc_row = acc_base + row;
+    const uint32_t bar_s_free = smem_u32(&bars->s_free);
     const uint32_t bar_p_lo = smem_u32(&bars->p_lo[t]);
     const uint32_t bar_p_hi = smem_u32(&bars->p_hi[t]);
 
@@ -579,30 +580,25 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
 
     bool ok = true;
     for (int j = 0; j < n_tiles && ok; ++j) {
-      // The MMA issuer pays ~100 cycles of idle tensor pipe for every barrier it polls, even a satisfied one,
-      // while this group spends a third of every iteration waiting for S.  So one thread of group 0 checks here
-      // that V_j and K_{j+1} have landed (they were requested two tiles ago); its arrival on the P barriers then
-      // carries that fact to the issuer, which uses V_j first in P_0(j) V_j and K_{j+1} first in Q_0 K_{j+1}^T.
-      bool kv_ok = true;
-      if (threadIdx.x == 0) {
-        const int iv = 2 * j + 1, ik = 2 * j + 2;
-        kv_ok = mbar_wait(smem_u32(&bars->kv_full[iv % kStages]), (iv / kStages) & 1, ctx, SITE_KV_FULL + iv % kStages);
-        if (kv_ok && j + 1 < n_tiles)
-          kv_ok = mbar_wait(smem_u32(&bars->kv_full[ik % kStages]), (ik / kStages) & 1, ctx, SITE_KV_FULL + ik % kStages);
-      }
-      ok = __all_sync(0xffffffffu, kv_ok && mbar_wait(smem_u32(&bars->s_full[t]), j & 1, ctx, SITE_S_FULL + t));
+      ok = warp_wait(&bars->s_full[t], j & 1, ctx, SITE_S_FULL + t);
       if (!ok) break;
       tc_fence_after();
       const int tile = tile_list != nullptr ? tile_list[tile_begin + j] : tile_begin + j;
       const int valid_cols = min(kv_eff - tile * kBlockN, kBlockN);
+      auto wait_pv = [&]() {
+        if (j == 0) return true;
+        const bool done = warp_wait(&bars->pv_done[t], (j - 1) & 1, ctx, SITE_O_FULL + t);
+        tc_fence_after();
+        return done;
+      };
       if (fixed_m) {
-        softmax_tile<true>(s_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_p_lo, bar_p_hi);
+        ok = softmax_tile<true>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
       } else {
-        softmax_tile<false>(s_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_p_lo, bar_p_hi);
+        ok = softmax_tile<false>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
       }
       o_live = true;
     }
-    if (ok) ok = warp_wait(&bars->o_full[t], 0, ctx, SITE_O_FULL + t);
+    if (ok) ok = warp_wait(&bars->pv_done[t], (n_tiles - 1) & 1, ctx, SITE_O_FULL + t);
     if (ok) {
       tc_fence_after();
       if (emit_state) {

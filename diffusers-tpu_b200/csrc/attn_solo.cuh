@@ -1,11 +1,12 @@
 // Joint-attention forward for sm_100a on 128-row query blocks: the kernel of attn_kernel.cuh on one query tile.
 //
-// The two softmax groups take alternate key tiles, S_t(j) = Q K_{2j+t}^T, each with its own (O_t, m, l); warp roles,
-// tensor memory and the order of the MMAs are those of the two-tile kernel, and group 0 merges (O_0, m, l) with
-// (O_1, m, l) at the end.  The period of the loop is the round trip of one S tile - softmax, P V, next Q K^T - as
-// it is with two query tiles, so a block is through its keys in half as many periods.  Taken for launches whose 256-row
-// blocks leave SMs idle or hold empty query tiles (solo_blocks in attn_api.cu).  It reads K and V once per 128
-// rows, through a ring of five slots (the second query tile's memory is the fifth).
+// The two softmax groups take alternate key tiles, S(e) = Q K_e^T for group e % 2, each with its own (O_t, m, l); warp
+// roles, tensor memory and barriers are those of the two-tile kernel, and group 0 merges (O_0, m, l) with
+// (O_1, m, l) at the end.  A block is through its keys in half as many periods of the loop.  Taken for launches whose
+// 256-row blocks leave SMs idle or hold empty query tiles (solo_blocks in attn_api.cu).  It reads K and V once per 128
+// rows, through a ring of six slots: with long keys the loads bound it (2 x 24 heads x 333 queries against 16731 keys
+// take 137 us, 148 without any exponentials or any MMAs in an earlier form; 157 with five slots and P written over S;
+// prefetching tiles to L2 some way ahead made it 4% slower).
 //
 // A kernel of its own rather than a case of the other: the two-tile kernel's loop is sensitive to its neighbourhood,
 // and as a template parameter of that body this form cost long sequences 2%.
@@ -17,7 +18,7 @@
 
 namespace dtb {
 
-constexpr int kSoloStages = 5;               // K/V ring slots
+constexpr int kSoloStages = 6;               // K/V ring slots
 constexpr int kSiteSoloReady = 70;           // beside WaitSite, reported in status[1] when a wait runs out
 
 struct __align__(8) SoloBarriers {
@@ -27,7 +28,8 @@ struct __align__(8) SoloBarriers {
   uint64_t s_full[2];
   uint64_t p_lo[2];         // first 64 keys of P_t written
   uint64_t p_hi[2];         // last 64 keys of P_t written
-  uint64_t o_full[2];
+  uint64_t pv_done[2];      // P_t V of a tile has run
+  uint64_t s_free;          // S has been read into registers
   uint64_t solo_ready;      // ml holds group 1's (m, l)
   float2 ml[kBlockM];
   uint32_t tmem_base;
@@ -115,8 +117,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
       mbar_init(smem_u32(&bars->s_full[i]), 1);
       mbar_init(smem_u32(&bars->p_lo[i]), kBlockM);
       mbar_init(smem_u32(&bars->p_hi[i]), kBlockM);
-      mbar_init(smem_u32(&bars->o_full[i]), 1);
+      mbar_init(smem_u32(&bars->pv_done[i]), 1);
     }
+    mbar_init(smem_u32(&bars->s_free), kBlockM);
     mbar_init(smem_u32(&bars->solo_ready), kBlockM);
     for (int i = 0; i < kSoloStages; ++i) {
       mbar_init(smem_u32(&bars->kv_full[i]), 1);
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  // Places in the K/V ring, in the order in which the issuer takes the tiles: K_0 K_1 V_0 K_2 V_1 ... K_{n-1} V_{n-2} V_{n-1}.
+  // Places in the K/V ring: K_0 K_1 V_0 K_2 V_1 ... K_{n-1} V_{n-2} V_{n-1}.
   auto place_k = [&](int e) { return e == 0 ? 0 : 2 * e - 1; };
   auto place_v = [&](int e) { return e == n_tiles - 1 ? 2 * n_tiles - 1 : 2 * e + 2; };
 
@@ -172,14 +175,11 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     }
     __syncwarp();
   } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------------ issuer of S(e) = Q K_e^T
     setmaxnreg_dec<kRegsService>();
     constexpr uint32_t idesc_qk = kQkFp8 ? make_idesc_e4m3(kBlockM, kBlockN) : make_idesc_bf16(kBlockM, kBlockN, false, false);
-    constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, kHeadDim, false, true);
     const uint64_t q_desc0 = make_smem_desc_sw128(smem_u32(smem_q), 16, 1024);
     const uint64_t k_desc0 = make_smem_desc_sw128(smem_u32(smem_kv), 16, 1024);
-    const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(smem_kv), kPanelBytes, 1024);
-    bool ok = true;
 
     auto issue_qk = [&](int t, int slot) {
       if (elect_one()) {
@@ -188,24 +188,45 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
 #pragma unroll
           for (int kk = 0; kk < kHeadDim / 32; ++kk) {   // 32 one-byte elements = 32 bytes of the swizzled row
             const uint64_t off = static_cast<uint64_t>((kk * 32) >> 4);
-            mma_ss_f8(tmem_base + t * kBlockN, q_desc0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
+            mma_ss_f8(tmem_base, q_desc0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
         } else {
 #pragma unroll
           for (int kk = 0; kk < kHeadDim / 16; ++kk) {
             const uint64_t off = static_cast<uint64_t>(((kk & 3) * 32 + (kk >> 2) * kPanelBytes) >> 4);
-            mma_ss(tmem_base + t * kBlockN, q_desc0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
+            mma_ss(tmem_base, q_desc0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
         }
         mma_commit(smem_u32(&bars->s_full[t]));
       }
       __syncwarp();
     };
+    auto commit_to = [&](uint64_t* bar) {
+      if (elect_one()) mma_commit(smem_u32(bar));
+      __syncwarp();
+    };
+
+    bool ok = warp_wait(&bars->q_full[0], 0, ctx, SITE_Q_FULL) && warp_wait(&bars->kv_full[0], 0, ctx, SITE_KV_FULL);
+    for (int e = 0; e < n_tiles && ok; ++e) {
+      const int slot = place_k(e) % kSoloStages;
+      if (e > 0) ok = warp_wait(&bars->s_free, (e - 1) & 1, ctx, SITE_S_FREE);
+      if (!ok) break;
+      tc_fence_after();
+      issue_qk(e & 1, slot);
+      commit_to(&bars->kv_empty[slot]);
+    }
+  } else if (warp == kPvWarp) {
+    // ------------------------------------------------------------------ issuer of O_t += P_t(e) V_e
+    setmaxnreg_dec<kRegsService>();
+    constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, kHeadDim, false, true);
+    const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(smem_kv), kPanelBytes, 1024);
+    bool ok = true;
+
     auto issue_pv = [&](int t, int slot, int half, bool accumulate) {
       if (elect_one()) {
         const uint64_t b0 = v_desc0 + static_cast<uint64_t>((slot * kTileBytes) >> 4);
         const uint32_t d_tmem = tmem_base + (kQTiles + t) * kBlockN;
-        const uint32_t a_tmem = tmem_base + t * kBlockN;
+        const uint32_t a_tmem = tmem_base + kBlockN + t * (kBlockN / 2);
 #pragma unroll
         for (int kk = half * 4; kk < half * 4 + 4; ++kk) {
           const uint64_t off = static_cast<uint64_t>((kk * 16 * 128) >> 4);
@@ -218,39 +239,19 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
       if (elect_one()) mma_commit(smem_u32(bar));
       __syncwarp();
     };
-    auto wait_kv = [&](int i) {
-      const int slot = i % kSoloStages;
-      return warp_wait(&bars->kv_full[slot], (i / kSoloStages) & 1, ctx, SITE_KV_FULL + slot);
-    };
-
-    // Prologue: S_t(0) = Q K_t^T.
-    ok = warp_wait(&bars->q_full[0], 0, ctx, SITE_Q_FULL);
-    for (int t = 0; t < min(n_tiles, 2) && ok; ++t) {
-      ok = wait_kv(t);
-      if (!ok) break;
-      tc_fence_after();
-      issue_qk(t, t);
-      commit_to(&bars->kv_empty[t]);
-    }
     const bool o_preloaded = kResidual && !p.acc_init;
-    // No wait for V_e or K_{e+2} here: the group of tile e checks both loads before it publishes P(e).
     for (int e = 0; e < n_tiles && ok; ++e) {
-      const int t = e & 1, j = e >> 1, vslot = place_v(e) % kSoloStages, kslot = place_k(e + 2) % kSoloStages;
+      const int t = e & 1, j = e >> 1, slot = place_v(e) % kSoloStages;
       ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);
       if (!ok) break;
       tc_fence_after();
-      issue_pv(t, vslot, 0, j > 0 || (o_preloaded && t == 0));
+      issue_pv(t, slot, 0, j > 0 || (o_preloaded && t == 0));
       ok = warp_wait(&bars->p_hi[t], j & 1, ctx, SITE_P_HI + t);
       if (!ok) break;
       tc_fence_after();
-      issue_pv(t, vslot, 1, true);
-      commit_to(&bars->kv_empty[vslot]);
-      if (e + 2 < n_tiles) {
-        issue_qk(t, kslot);
-        commit_to(&bars->kv_empty[kslot]);
-      } else {
-        commit_to(&bars->o_full[t]);
-      }
+      issue_pv(t, slot, 1, true);
+      commit_to(&bars->pv_done[t]);
+      commit_to(&bars->kv_empty[slot]);
     }
   } else if (warp < kMmaWarp) {
     // ------------------------------------------------------------------ softmax groups
@@ -259,11 +260,13 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     const int row_in_tile = threadIdx.x & (kBlockM - 1);
     const int row = q0 + row_in_tile;  // query row within this call
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_tmem = tmem_base + lane_off + t * kBlockN;
+    const uint32_t s_tmem = tmem_base + lane_off;
+    const uint32_t p_tmem = tmem_base + lane_off + kBlockN + t * (kBlockN / 2);
     const uint32_t o_tmem = tmem_base + lane_off + (kQTiles + t) * kBlockN;
     const float scale_log2 = p.scale_log2;
     const bool row_in_range = row < p.Sq;
     const int64_t acc_row = acc_base + row;
+    const uint32_t bar_s_free = smem_u32(&bars->s_free);
     const uint32_t bar_p_lo = smem_u32(&bars->p_lo[t]);
     const uint32_t bar_p_hi = smem_u32(&bars->p_hi[t]);
 
@@ -327,16 +330,16 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     const int n_own = (n_tiles + 1 - t) >> 1;   // key tiles of this group
     for (int j = 0; j < n_own && ok; ++j) {
       const int e = 2 * j + t;
-      // One thread checks that V_e and K_{e+2} have landed; its arrival on the P barriers carries that to the issuer.
-      // It does so after the wait for S(e), not before: a parity wait for one use of a ring slot also returns while
-      // the use before it is still in flight, so that use has to be known complete.  V_e follows K_{e-1} in its slot
-      // (the last V follows V_{n-4}), which the other group checked for its P(e-3), and that group may be a tile behind;
-      // but S(e) is issued after P(e-3) V_{e-3}.  K_{e+2} follows V_{e-2}, which this thread checked itself.
+      // One thread checks that V_e and K_{e+1} have landed; its arrivals on s_free and the P barriers carry that to the
+      // issuers.  It does so after the wait for S(e), not before: a parity wait for one use of a ring slot also returns
+      // while the use before it is still in flight, so that use has to be known complete.  V_e follows V_{e-3} in its slot,
+      // which the other group checked for its tile e-3, before it read S(e-1), and S(e) is issued after that;
+      // K_{e+1} follows K_{e-2}, which S(e-2) was made of.
       bool landed = mbar_wait(smem_u32(&bars->s_full[t]), j & 1, ctx, SITE_S_FULL + t);
       if (landed && row_in_tile == 0) {
-        const int iv = place_v(e), ik = place_k(e + 2);
+        const int iv = place_v(e), ik = place_k(e + 1);
         landed = mbar_wait(smem_u32(&bars->kv_full[iv % kSoloStages]), (iv / kSoloStages) & 1, ctx, SITE_KV_FULL + iv % kSoloStages);
-        if (landed && e + 2 < n_tiles)
+        if (landed && e + 1 < n_tiles)
           landed = mbar_wait(smem_u32(&bars->kv_full[ik % kSoloStages]), (ik / kSoloStages) & 1, ctx, SITE_KV_FULL + ik % kSoloStages);
       }
       ok = __all_sync(0xffffffffu, landed);
@@ -344,14 +347,20 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
       tc_fence_after();
       const int tile = tile_list != nullptr ? tile_list[e] : e;
       const int valid_cols = min(kv_eff - tile * kBlockN, kBlockN);
+      auto wait_pv = [&]() {
+        if (j == 0) return true;
+        const bool done = warp_wait(&bars->pv_done[t], (j - 1) & 1, ctx, SITE_O_FULL + t);
+        tc_fence_after();
+        return done;
+      };
       if (fixed_m) {
-        softmax_tile<true>(s_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_p_lo, bar_p_hi);
+        ok = softmax_tile<true>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
       } else {
-        softmax_tile<false>(s_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_p_lo, bar_p_hi);
+        ok = softmax_tile<false>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
       }
       o_live = true;
     }
-    if (ok && n_own > 0) ok = warp_wait(&bars->o_full[t], 0, ctx, SITE_O_FULL + t);
+    if (ok && n_own > 0) ok = warp_wait(&bars->pv_done[t], (n_own - 1) & 1, ctx, SITE_O_FULL + t);
     // Group 1 hands over its (m, l); its O is read by group 0's warps, which see the same lanes.
     float w_own = 1.f, w_other = 1.f;      // factors of O_0 and O_1
     const bool merge = n_tiles > 1;
@@ -361,7 +370,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
         *ml = make_float2(m_used, l_sum);
         mbar_arrive(smem_u32(&bars->solo_ready));
       } else {
-        ok = warp_wait(&bars->solo_ready, 0, ctx, kSiteSoloReady) && warp_wait(&bars->o_full[1], 0, ctx, SITE_O_FULL + 1);
+        ok = warp_wait(&bars->solo_ready, 0, ctx, kSiteSoloReady) && warp_wait(&bars->pv_done[1], ((n_tiles >> 1) - 1) & 1, ctx, SITE_O_FULL + 1);
         if (ok) {
           // A group whose sum is 0 has no say in the offset.  Any other sum has, NaN included, and both accumulators are
           // always taken: what is not finite in either half of the keys shows in the output, as with one group.
