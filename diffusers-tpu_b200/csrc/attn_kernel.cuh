@@ -147,12 +147,15 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const 
 // The whole S row comes out of tensor memory in one load, after which S belongs to the other group; the row max uses
 // three-input max; the scale-and-subtract and the row sum run on packed f32 pairs; P goes to tensor memory in two halves
 // of 64 keys, each published on its own mbarrier so the PV MMA of the first half runs while the second half is still
-// being exponentiated.  wait_pv() returns when the P V of the group's tile before has run; with online softmax it stands in front
-// of the exponentials so that the first 32 probabilities can be stored under them (behind them: 371 -> 393 us on the
-// 1024-pixel shape).  Returns false when a wait ran out.  Exponentiating the first half before the maximum is known, which paid
-// while the next Q K^T waited for P, costs 6% now (371 -> 394 us).
+// being exponentiated.  wait_pv() returns when the P V of the group's tile before has run; it stands in front of
+// the exponentials, so that the first 32 probabilities can be stored under those of the next 32.  (Behind the first 64, 2 x 24
+// x 4608 rows: online 371 -> 393 us, a bounded call with its smoothing and norms 464 -> 478.)  With two query tiles it also
+// stands in front of the maximum (kWaitFirst: E4M3 scores 2 x 24 x 16896 4890 us, 5040 behind it; 2 x 24 x 4608 412, 415);
+// with one, where loads set the pace, behind it (333 queries against 16731 keys 158 us, 166 in front).  Returns false when a
+// wait ran out.  Exponentiating the first half before the maximum is known, which paid while the next Q K^T waited for P,
+// costs 6% now (371 -> 394 us).
 // ---------------------------------------------------------------------------
-template <bool kFixedM, class WaitPv>
+template <bool kFixedM, bool kWaitFirst, class WaitPv>
 __device__ __forceinline__ bool softmax_tile(uint32_t s_tmem, uint32_t p_tmem, uint32_t o_tmem, float scale_log2, int valid_cols,
                                              bool o_live, float& m_used, float& l_sum, uint32_t bar_s_free, uint32_t bar_p_lo,
                                              uint32_t bar_p_hi, WaitPv wait_pv) {
@@ -169,7 +172,7 @@ __device__ __forceinline__ bool softmax_tile(uint32_t s_tmem, uint32_t p_tmem, u
   uint64_t acc2 = pack_f32x2(0.f, 0.f);
   uint32_t pk[32];
   // 2^(s * scale - m) for 64 keys: packed into pk, summed into acc2.
-  auto exp_half = [&](int half, bool store_first) {
+  auto exp_half = [&](int half) {
     const uint64_t neg_m2 = pack_f32x2(-m_used, -m_used);
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
@@ -183,11 +186,10 @@ __device__ __forceinline__ bool softmax_tile(uint32_t s_tmem, uint32_t p_tmem, u
       pk[i] = pack_bf16x2(p0, p1);
       // The first 32 keys of the half go to tensor memory while the other 32 are exponentiated, which hides half
       // of the store's latency.  Nothing reads them before the arrive in publish().
-      if (store_first && i == 15) tmem_st16(p_tmem + half * 32, pk);
+      if (i == 15) tmem_st16(p_tmem + half * 32, pk);
     }
   };
-  auto publish = [&](int half, bool first_stored) {
-    if (!first_stored) tmem_st16(p_tmem + half * 32, pk);
+  auto publish = [&](int half) {
     tmem_st16(p_tmem + half * 32 + 16, pk + 16);
     tmem_wait_st();
     tc_fence_before();
@@ -206,10 +208,11 @@ __device__ __forceinline__ bool softmax_tile(uint32_t s_tmem, uint32_t p_tmem, u
     return fmaxf(max3(mxs[0], mxs[1], mxs[2]), fmaxf(max3(mxs[3], mxs[4], mxs[5]), fmaxf(mxs[6], mxs[7]))) * scale_log2;
   };
 
+  if ((kWaitFirst || kFixedM) && !wait_pv()) return false;
   if (!kFixedM) {
     const float mx = row_max();
     const bool grow = mx > m_used + kRescaleThreshold;  // always true while m_used is -inf or kLowestOffset, for finite logits
-    if (!wait_pv()) return false;
+    if (!kWaitFirst && !wait_pv()) return false;
     if (o_live && __any_sync(0xffffffffu, grow)) {
       const float alpha = grow ? ex2(m_used - mx) : 1.0f;
       l_sum *= alpha;
@@ -227,15 +230,11 @@ __device__ __forceinline__ bool softmax_tile(uint32_t s_tmem, uint32_t p_tmem, u
       l_sum *= ex2(m_used - mx);
     }
     if (grow) m_used = mx;
-    exp_half(0, true);
-    publish(0, true);
-  } else {
-    exp_half(0, false);
-    if (!wait_pv()) return false;
-    publish(0, false);
   }
-  exp_half(1, true);
-  publish(1, true);
+  exp_half(0);
+  publish(0);
+  exp_half(1);
+  publish(1);
   float a0, a1;
   unpack_f32x2(acc2, a0, a1);
   l_sum += a0 + a1;
@@ -592,9 +591,9 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
         return done;
       };
       if (fixed_m) {
-        ok = softmax_tile<true>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
+        ok = softmax_tile<true, true>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
       } else {
-        ok = softmax_tile<false>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
+        ok = softmax_tile<false, true>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
       }
       o_live = true;
     }

@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
         return done;
       };
       if (fixed_m) {
-        ok = softmax_tile<true>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
+        ok = softmax_tile<true, false>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
       } else {
-        ok = softmax_tile<false>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
+        ok = softmax_tile<false, false>(s_tmem, p_tmem, o_tmem, scale_log2, valid_cols, o_live, m_used, l_sum, bar_s_free, bar_p_lo, bar_p_hi, wait_pv);
       }
       o_live = true;
     }
