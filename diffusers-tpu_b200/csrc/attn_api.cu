@@ -307,6 +307,12 @@ constexpr int kMinPieceTiles = 4;      // no run shorter than this many key tile
 #endif
 constexpr int kPieceOverheadTiles = DTB_PIECE_OVERHEAD_TILES;
 
+// What it costs more, beside 128-row blocks, where there are more pieces than SMs, so that some SM sweeps two.  Device time,
+// pieces / 128-row blocks: 1 x 3 heads x 4608 rows (14 + 13 key-tile times by the plan, 30 measured) 45.0 / 36.3 us, 1 x 3 x
+// 3072 34.3 / 26.1, 1 x 4 x 3072 36.4 / 26.2, 1 x 3 x 5200 53.3 / 43.0, 1 x 2 x 9216 85.1 / 74.3; with fewer pieces the plan
+// holds: 1 x 1 x 3072 19.2 / 25.8, 1 x 2 x 3072 22.7 / 26.1, 1 x 1 x 9216 51.6 / 64.8.
+constexpr int kSecondPieceTiles = 3;
+
 // Key-tile times that a block costs beyond its key tiles: launch, pipeline fill and drain, epilogue.
 constexpr int kBlockOverheadTiles = 5;
 
@@ -362,9 +368,6 @@ void plan_balanced(const dtb_attn_params* p, int sms, BalancedPlan* plan) {
   if (runs <= tail) return;
   const long long run_len = (tiles + runs - 1) / runs;
   if (run_len + kPieceOverheadTiles > n) return;   // the plain launch is as fast or faster
-  // ... and so may be 128-row blocks, where there are few blocks.  (The pieces' overhead is taken as all that they cost
-  // here, not as what they cost beyond a block's own start and finish: where the two are close, the pieces stay.)
-  if (solo_beats(p, sms, n, units / sms * (n + kBlockOverheadTiles) + run_len + kPieceOverheadTiles)) return;
   struct Piece { int x, tb, te; };
   Piece pieces[kMaxPieces];
   int np = 0;
@@ -378,6 +381,10 @@ void plan_balanced(const dtb_attn_params* p, int sms, BalancedPlan* plan) {
       s0 = end;
     }
   }
+  // ... and so may be 128-row blocks, where there are few blocks.  (The pieces' overhead is taken as all that they cost
+  // here, not as what they cost beyond a block's own start and finish: where the two are close, the pieces stay.)
+  const int second = np > sms ? kSecondPieceTiles : 0;
+  if (solo_beats(p, sms, n, units / sms * (n + kBlockOverheadTiles) + run_len + kPieceOverheadTiles + second)) return;
   // slots: consecutive per unit, in the order of the key ranges (pieces are generated in that order)
   PieceMerge& mg = plan->merge;
   mg.first_unit = static_cast<int>(units - tail);
