@@ -333,11 +333,11 @@ long long plain_time(const dtb_attn_params* p, int sms, int rows, long long n) {
 
 // Whether `time` is worse than a launch of 128-row blocks.  Those read K and V once per 128 rows instead of once per
 // 256, which is paid for out of the margin.  Measured, 256-row blocks against 128-row ones, device time:
-//   one round each: 54 / 108 blocks x 18 tiles 34.6 / 23.6 us; 72 / 144 x 36 60.8 / 39.6; 96 / 144 x 132 221 / 157
-//   two rounds against three: 198 / 396 x 132 441 / 423 us in a loop of seconds, under the power limit (a ring step
-//   with that many 455 / 428, with E4M3 scores 441 / 383); 216 / 432 x 36 123 / 117, a model ratio of 0.84, left out
-//   the same with few tiles, as under a narrow table: 222 / 444 x 6 34.0 / 38.1 us, x 12 53.4 / 55.0, x 24 90.0 / 88.0
-//   one against two: 108 / 216 x 36 61.8 / 74.9 us
+//   one round each: 54 / 108 blocks x 18 tiles 31.7 / 21.6 us; 72 / 144 x 36 57.4 / 41.8; 96 / 144 x 132 219 / 159
+//   two rounds against three: 198 / 396 x 132 420 / 410 us in a loop of half a second, under the power limit; 216 / 432 x
+//   36 125 / 124, a model ratio of 0.84, left out
+//   the same with few tiles, as under a narrow table (with P written over S): 222 / 444 x 6 34.0 / 38.1 us, x 12 53.4 / 55.0, x 24 90.0 / 88.0
+//   one against two: 108 / 216 x 36 62.6 / 74.6 us
 bool solo_beats(const dtb_attn_params* p, int sms, int n, long long time) {
   return 5 * plain_time(p, sms, kBlockM, n) < 4 * time;
 }
