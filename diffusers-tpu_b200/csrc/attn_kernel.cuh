@@ -383,6 +383,9 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
   // Places in the K/V ring, in the order in which the issuer takes the tiles: K_0 K_1 V_0 K_2 V_1 ... K_{n-1} V_{n-2} V_{n-1}.
   auto place_k = [&](int e) { return e == 0 ? 0 : 2 * e - 1; };
   auto place_v = [&](int e) { return e == n_tiles - 1 ? 2 * n_tiles - 1 : 2 * e + 2; };
+  // Whether the producer waits for the slot of place i to be free.  Nobody waits for the others, and an arrival that nobody
+  // waits for may come when the block is gone and its shared memory another block's: they are not committed to.
+  auto reloaded = [&](int i) { return i + kStages < 2 * n_tiles; };
 
   if (warp == kLoadWarp) {
     // ------------------------------------------------------------------ TMA producer
@@ -460,7 +463,7 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
         if (!ok) break;
         tc_fence_after();
         issue_qk(t, slot);
-        if (t == kQTiles - 1) commit_to(&bars->kv_empty[slot]);
+        if (t == kQTiles - 1 && reloaded(i)) commit_to(&bars->kv_empty[slot]);
       }
     }
   } else if (warp == kPvWarp) {
@@ -500,7 +503,7 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
         tc_fence_after();
         issue_pv(t, slot, 1, true);
         commit_to(&bars->pv_done[t]);
-        if (t == kQTiles - 1) commit_to(&bars->kv_empty[slot]);
+        if (t == kQTiles - 1 && reloaded(i)) commit_to(&bars->kv_empty[slot]);
       }
     }
   } else if (warp < kMmaWarp) {

@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
   // Places in the K/V ring: K_0 K_1 V_0 K_2 V_1 ... K_{n-1} V_{n-2} V_{n-1}.
   auto place_k = [&](int e) { return e == 0 ? 0 : 2 * e - 1; };
   auto place_v = [&](int e) { return e == n_tiles - 1 ? 2 * n_tiles - 1 : 2 * e + 2; };
+  auto reloaded = [&](int i) { return i + kSoloStages < 2 * n_tiles; };   // as in the two-tile kernel
 
   if (warp == kLoadWarp) {
     // ------------------------------------------------------------------ TMA producer
@@ -208,12 +209,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
 
     bool ok = warp_wait(&bars->q_full[0], 0, ctx, SITE_Q_FULL) && warp_wait(&bars->kv_full[0], 0, ctx, SITE_KV_FULL);
     for (int e = 0; e < n_tiles && ok; ++e) {
-      const int slot = place_k(e) % kSoloStages;
+      const int i = place_k(e), slot = i % kSoloStages;
       if (e > 0) ok = warp_wait(&bars->s_free, (e - 1) & 1, ctx, SITE_S_FREE);
       if (!ok) break;
       tc_fence_after();
       issue_qk(e & 1, slot);
-      commit_to(&bars->kv_empty[slot]);
+      if (reloaded(i)) commit_to(&bars->kv_empty[slot]);
     }
   } else if (warp == kPvWarp) {
     // ------------------------------------------------------------------ issuer of O_t += P_t(e) V_e
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     };
     const bool o_preloaded = kResidual && !p.acc_init;
     for (int e = 0; e < n_tiles && ok; ++e) {
-      const int t = e & 1, j = e >> 1, slot = place_v(e) % kSoloStages;
+      const int t = e & 1, j = e >> 1, i = place_v(e), slot = i % kSoloStages;
       ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);
       if (!ok) break;
       tc_fence_after();
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
       tc_fence_after();
       issue_pv(t, slot, 1, true);
       commit_to(&bars->pv_done[t]);
-      commit_to(&bars->kv_empty[slot]);
+      if (reloaded(i)) commit_to(&bars->kv_empty[slot]);
     }
   } else if (warp < kMmaWarp) {
     // ------------------------------------------------------------------ softmax groups

@@ -7,8 +7,9 @@ the order of their issuer at any time after it has issued them.  An mbarrier is 
 still waits for and its outstanding bytes, so a parity wait can pass one use early or block for ever as the real one does.
 
 One run of the programs says which write each access to S, P, O, Q, a slot of the K/V ring or the exchanged row statistics
-follows, and that the accumulators come out as the sums over the right tiles; every other interleaving has to agree.  Small
-mistakes planted in a copy of the sources, one at a time, have to be found.
+follows, and that the accumulators come out as the sums over the right tiles; every other interleaving has to agree, and at the
+end of a block nothing may still be in flight to its shared memory.  Small mistakes planted in a copy of the sources, one at
+a time, have to be found.
 
 Not covered: the 128 threads of a group are two, warps run one instruction stream (no divergence), waits do not run out."""
 import functools
@@ -308,6 +309,8 @@ class Block:
         while stack:
             state = stack.pop()
             if self.ended(state):
+                if self.in_flight(state):
+                    raise Wrong("in flight at the end of the block")
                 continue
             moved = False
             for after in self.steps(state):
@@ -377,6 +380,8 @@ MISTAKES = {
     "pair: K not waited for": ("pair", PAIR, "const int i = place_k(j), slot = i % kStages;\n      for (int t = 0; t < kQTiles && ok; ++t) {\n        if (j == 0) ok = warp_wait(&bars->q_full[t], 0, ctx, SITE_Q_FULL + t);\n        if (ok && t == 0)", "const int i = place_k(j), slot = i % kStages;\n      for (int t = 0; t < kQTiles && ok; ++t) {\n        if (j == 0) ok = warp_wait(&bars->q_full[t], 0, ctx, SITE_Q_FULL + t);\n        if (false)"),
     "pair: Q not waited for": ("pair", PAIR, "if (j == 0) ok = warp_wait(&bars->q_full[t], 0", "if (j == 0) ok = t == 1 || warp_wait(&bars->q_full[t], 0"),
     "pair: K given back a query tile early": ("pair", PAIR, "issue_qk(t, slot);\n        if (t == kQTiles - 1", "issue_qk(t, slot);\n        if (t == 0"),
+    "pair: arrivals that nobody waits for": ("pair", PAIR, "return i + kStages < 2 * n_tiles;", "return true;"),
+    "pair: a slot that is reloaded is not given back": ("pair", PAIR, "return i + kStages < 2 * n_tiles;", "return i + kStages + 1 < 2 * n_tiles;"),
     # P V of the two-tile kernel
     "pair: V not waited for": ("pair", PAIR, "const int i = place_v(j), slot = i % kStages;\n      for (int t = 0; t < kQTiles && ok; ++t) {\n        if (t == 0)", "const int i = place_v(j), slot = i % kStages;\n      for (int t = 0; t < kQTiles && ok; ++t) {\n        if (false)"),
     "pair: first half of P not waited for": ("pair", PAIR, "if (ok) ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);", ""),
@@ -394,6 +399,7 @@ MISTAKES = {
     "pair: no fence behind the wait for the last P V": ("pair", PAIR, "ctx, SITE_O_FULL + t);\n    if (ok) {\n      tc_fence_after();", "ctx, SITE_O_FULL + t);\n    if (ok) {"),
     "softmax: P published before it is written": ("pair", PAIR, "    tmem_st16(p_tmem + half * 32 + 16, pk + 16);\n    tmem_wait_st();\n    tc_fence_before();\n    mbar_arrive(half == 0 ? bar_p_lo : bar_p_hi);", "    tc_fence_before();\n    mbar_arrive(half == 0 ? bar_p_lo : bar_p_hi);\n    tmem_st16(p_tmem + half * 32 + 16, pk + 16);\n    tmem_wait_st();\n    tc_fence_before();"),
     # the one-tile kernel
+    "solo: arrivals that nobody waits for": ("solo", SOLO, "return i + kSoloStages < 2 * n_tiles;", "return true;"),
     "solo: S overwritten before it is read": ("solo", SOLO, "if (e > 0) ok = warp_wait(&bars->s_free, (e - 1) & 1, ctx, SITE_S_FREE);", ""),
     "solo: V not checked": ("solo", SOLO, "landed = mbar_wait(smem_u32(&bars->kv_full[iv % kSoloStages]), (iv / kSoloStages) & 1, ctx, SITE_KV_FULL + iv % kSoloStages);", ""),
     "solo: K not checked": ("solo", SOLO, "landed = mbar_wait(smem_u32(&bars->kv_full[ik % kSoloStages]), (ik / kSoloStages) & 1, ctx, SITE_KV_FULL + ik % kSoloStages);", ";"),
