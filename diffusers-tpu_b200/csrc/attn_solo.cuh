@@ -4,9 +4,13 @@
 // roles, tensor memory and barriers are those of the two-tile kernel, and group 0 merges (O_0, m, l) with
 // (O_1, m, l) at the end.  A block is through its keys in half as many periods of the loop.  Taken for launches whose
 // 256-row blocks leave SMs idle or hold empty query tiles (solo_blocks in attn_api.cu).  It reads K and V once per 128
-// rows, through a ring of six slots: with long keys the loads bound it (2 x 24 heads x 333 queries against 16731 keys
-// take 137 us, 148 without any exponentials or any MMAs in an earlier form; 157 with five slots and P written over S;
-// prefetching tiles to L2 some way ahead made it 4% slower).
+// rows, through a ring of six slots: with long keys the loads bound it, 8 TB/s out of L2.
+//
+// The issuers wait for the loads.  While each group had an S of its own, one of its threads did, in the time that it waited for
+// S; with one S those checks stand between the arrival of S and its read, in the chain that sets the pace.  Device time of
+// calls in short loops, P over S / one S, checks in the groups / checks in the issuers: 1 x 3 heads x 1280 rows against 32 key
+// tiles 33.8 / 32.1 / 30.1 us, with bounded logits 32.4 / 32.4 / 28.7, as a partial state 34.5 / 37.4 / 30.8, by a table 35.6 /
+// 37.0 / 31.3; 2 x 24 x 333 queries against 16731 keys 158.3 / 144.4 / 135.7.
 //
 // A kernel of its own rather than a case of the other: the two-tile kernel's loop is sensitive to its neighbourhood,
 // and as a template parameter of that body this form cost long sequences 2%.
@@ -207,10 +211,11 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
       __syncwarp();
     };
 
-    bool ok = warp_wait(&bars->q_full[0], 0, ctx, SITE_Q_FULL) && warp_wait(&bars->kv_full[0], 0, ctx, SITE_KV_FULL);
+    bool ok = warp_wait(&bars->q_full[0], 0, ctx, SITE_Q_FULL);
     for (int e = 0; e < n_tiles && ok; ++e) {
       const int i = place_k(e), slot = i % kSoloStages;
-      if (e > 0) ok = warp_wait(&bars->s_free, (e - 1) & 1, ctx, SITE_S_FREE);
+      ok = warp_wait(&bars->kv_full[slot], (i / kSoloStages) & 1, ctx, SITE_KV_FULL + slot);
+      if (ok && e > 0) ok = warp_wait(&bars->s_free, (e - 1) & 1, ctx, SITE_S_FREE);
       if (!ok) break;
       tc_fence_after();
       issue_qk(e & 1, slot);
@@ -243,7 +248,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     const bool o_preloaded = kResidual && !p.acc_init;
     for (int e = 0; e < n_tiles && ok; ++e) {
       const int t = e & 1, j = e >> 1, i = place_v(e), slot = i % kSoloStages;
-      ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);
+      ok = warp_wait(&bars->kv_full[slot], (i / kSoloStages) & 1, ctx, SITE_KV_FULL + slot);
+      if (ok) ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);
       if (!ok) break;
       tc_fence_after();
       issue_pv(t, slot, 0, j > 0 || (o_preloaded && t == 0));
@@ -331,19 +337,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_solo_kernel(const __grid_
     const int n_own = (n_tiles + 1 - t) >> 1;   // key tiles of this group
     for (int j = 0; j < n_own && ok; ++j) {
       const int e = 2 * j + t;
-      // One thread checks that V_e and K_{e+1} have landed; its arrivals on s_free and the P barriers carry that to the
-      // issuers.  It does so after the wait for S(e), not before: a parity wait for one use of a ring slot also returns
-      // while the use before it is still in flight, so that use has to be known complete.  V_e follows V_{e-3} in its slot,
-      // which the other group checked for its tile e-3, before it read S(e-1), and S(e) is issued after that;
-      // K_{e+1} follows K_{e-2}, which S(e-2) was made of.
-      bool landed = mbar_wait(smem_u32(&bars->s_full[t]), j & 1, ctx, SITE_S_FULL + t);
-      if (landed && row_in_tile == 0) {
-        const int iv = place_v(e), ik = place_k(e + 1);
-        landed = mbar_wait(smem_u32(&bars->kv_full[iv % kSoloStages]), (iv / kSoloStages) & 1, ctx, SITE_KV_FULL + iv % kSoloStages);
-        if (landed && e + 1 < n_tiles)
-          landed = mbar_wait(smem_u32(&bars->kv_full[ik % kSoloStages]), (ik / kSoloStages) & 1, ctx, SITE_KV_FULL + ik % kSoloStages);
-      }
-      ok = __all_sync(0xffffffffu, landed);
+      ok = warp_wait(&bars->s_full[t], j & 1, ctx, SITE_S_FULL + t);
       if (!ok) break;
       tc_fence_after();
       const int tile = tile_list != nullptr ? tile_list[e] : e;

@@ -372,6 +372,16 @@ def test_every_form_and_softmax_is_ordered_and_ends(built, form, mode, state, n,
     assert _run(built(), form, n, mode, state, warps) is None
 
 
+@pytest.mark.parametrize("form", ["pair", "pair8", "pieces", "solo", "solo8"])
+@pytest.mark.parametrize("mode", ["growing", "bounded"])
+def test_nothing_stands_between_s_and_its_read(built, form, mode):
+    """A group that has seen its S gives it back before it waits for anything else: the next Q K^T depends on that."""
+    roles, names, _ = _trace(built(), form, 6, mode, "fresh")
+    for role in [r for r in roles if r.startswith("group")]:
+        order = [names[e[1]] for e in roles[role] if e[0] in ("wait", "arrive")]
+        assert all(after == "s_free" for before, after in zip(order, order[1:]) if before == "s_full"), role
+
+
 PAIR, SOLO = "attn_kernel.cuh", "attn_solo.cuh"
 MISTAKES = {
     # Q K^T of the two-tile kernel
@@ -400,10 +410,10 @@ MISTAKES = {
     "softmax: P published before it is written": ("pair", PAIR, "    tmem_st16(p_tmem + half * 32 + 16, pk + 16);\n    tmem_wait_st();\n    tc_fence_before();\n    mbar_arrive(half == 0 ? bar_p_lo : bar_p_hi);", "    tc_fence_before();\n    mbar_arrive(half == 0 ? bar_p_lo : bar_p_hi);\n    tmem_st16(p_tmem + half * 32 + 16, pk + 16);\n    tmem_wait_st();\n    tc_fence_before();"),
     # the one-tile kernel
     "solo: arrivals that nobody waits for": ("solo", SOLO, "return i + kSoloStages < 2 * n_tiles;", "return true;"),
-    "solo: S overwritten before it is read": ("solo", SOLO, "if (e > 0) ok = warp_wait(&bars->s_free, (e - 1) & 1, ctx, SITE_S_FREE);", ""),
-    "solo: V not checked": ("solo", SOLO, "landed = mbar_wait(smem_u32(&bars->kv_full[iv % kSoloStages]), (iv / kSoloStages) & 1, ctx, SITE_KV_FULL + iv % kSoloStages);", ""),
-    "solo: K not checked": ("solo", SOLO, "landed = mbar_wait(smem_u32(&bars->kv_full[ik % kSoloStages]), (ik / kSoloStages) & 1, ctx, SITE_KV_FULL + ik % kSoloStages);", ";"),
-    "solo: first half of P not waited for": ("solo", SOLO, "ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);", ""),
+    "solo: S overwritten before it is read": ("solo", SOLO, "if (ok && e > 0) ok = warp_wait(&bars->s_free, (e - 1) & 1, ctx, SITE_S_FREE);", ""),
+    "solo: V not waited for": ("solo", SOLO, "ok = warp_wait(&bars->kv_full[slot], (i / kSoloStages) & 1, ctx, SITE_KV_FULL + slot);\n      if (ok) ok = warp_wait(&bars->p_lo", "if (ok) ok = warp_wait(&bars->p_lo"),
+    "solo: K not waited for": ("solo", SOLO, "ok = warp_wait(&bars->kv_full[slot], (i / kSoloStages) & 1, ctx, SITE_KV_FULL + slot);\n      if (ok && e > 0)", "if (ok && e > 0)"),
+    "solo: first half of P not waited for": ("solo", SOLO, "if (ok) ok = warp_wait(&bars->p_lo[t], j & 1, ctx, SITE_P_FULL + t);", ""),
     "solo: second half of P not waited for": ("solo", SOLO, "ok = warp_wait(&bars->p_hi[t], j & 1, ctx, SITE_P_HI + t);", ""),
     "solo: P written before the last P V": ("solo", SOLO, "if (j == 0) return true;", "return true;"),
     "solo: slot reloaded before it is free": ("solo", SOLO, "if (use > 0) ok = mbar_wait(smem_u32(&bars->kv_empty[slot]), (use - 1) & 1, ctx, SITE_KV_EMPTY + slot);", ""),
@@ -416,13 +426,3 @@ MISTAKES = {
 def test_a_planted_mistake_is_found(built, mistake):
     form, *edit = MISTAKES[mistake]
     assert any(_run(built(tuple(edit)), form, n, "growing") for n in (4, 5))
-
-
-def test_the_groups_may_check_loads_before_s(built):
-    """A parity wait for one use of a slot passes while the use before it is in flight.  That use is known complete either way: V_{e-3} was
-    checked before the other group gave S(e-3) back, ahead of S(e-2), and K_{e-2} made S(e-2), which the group has read."""
-    edit = (SOLO, "bool landed = mbar_wait(smem_u32(&bars->s_full[t]), j & 1, ctx, SITE_S_FULL + t);\n      if (landed && row_in_tile == 0) {",
-            "bool landed = true;\n      if (row_in_tile == 0) {", "ok = __all_sync(0xffffffffu, landed);",
-            "ok = __all_sync(0xffffffffu, landed && mbar_wait(smem_u32(&bars->s_full[t]), j & 1, ctx, SITE_S_FULL + t));")
-    for n in (4, 7, 8):
-        assert _run(built(edit), "solo", n) is None
