@@ -331,6 +331,14 @@ __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
 }
 
+// Eight consecutive words of global memory in one 32-byte load; the address has to be a multiple of 32.
+__device__ __forceinline__ void ld_global8(const float* src, uint32_t* r) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "l"(src)
+               : "memory");
+}
+
 // ----------------------------------------------------------------------------
 // Math helpers
 // ----------------------------------------------------------------------------

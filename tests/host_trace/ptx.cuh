@@ -117,6 +117,7 @@ inline void mma_commit(uint32_t bar) { record("commit %u\n", bar); }
 template <int kRegs> void setmaxnreg_inc() {}
 template <int kRegs> void setmaxnreg_dec() {}
 
+inline void ld_global8(const float* src, uint32_t* r) { std::memcpy(r, src, 32); }
 inline float ex2(float x) { return std::exp2(x); }
 inline uint64_t pack_f32x2(float lo, float hi) { return static_cast<uint64_t>(__float_as_uint(hi)) << 32 | __float_as_uint(lo); }
 inline void unpack_f32x2(uint64_t v, float& lo, float& hi) {

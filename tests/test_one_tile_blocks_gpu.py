@@ -121,3 +121,26 @@ def test_128_row_blocks_over_131_key_tiles():
     assert _block_rows(q.to(DEV), k.to(DEV)) == 128
     out = dtb200.attention(q.to(DEV), k.to(DEV), v.to(DEV), kv_len=[16700], zero_padded_rows=False)
     _check(out, O.attention_fp32(q, k, v, kv_len=[16700], zero_padded_rows=False))
+
+
+@pytest.mark.parametrize("words", [4, 8, 12])
+@pytest.mark.parametrize("Sq", [77, 300])
+@pytest.mark.parametrize("second", ["online", "bounded", "e4m3"])
+def test_a_running_state_may_start_at_any_multiple_of_16_bytes(words, Sq, second):
+    """128-row blocks read it 32 bytes at a time where it allows that and 16 where not: the same state either way."""
+    q, k, v = (t.to(DEV) for t in _inputs(1, 2, Sq, 2048, seed=Sq))
+    mk = dtb200.fixed_m_operands(q, k) if second == "bounded" else None
+    states = []
+    for at in (0, words):
+        state = dtb200.ResidualState(1, 2, Sq, q.device)
+        state.o = torch.full((2 * Sq * 128 + 16,), float("nan"), device=DEV)[at:at + 2 * Sq * 128].view(1, 2, Sq, 128)
+        assert state.o.data_ptr() % 64 == 4 * at and _block_rows(q, k[:, :, :1024]) == 128
+        # after an online step the bounded one finds a state relative to another offset than its own
+        dtb200.residual_attention_(state, q, k[:, :, :1024], v[:, :, :1024])
+        dtb200.residual_attention_(state, q, k[:, :, 1024:], v[:, :, 1024:], kv_offset=1024, use_fixed_m=second == "bounded", mk=mk,
+                                   qk_fp8=second == "e4m3")
+        states.append(state)
+    dtb200.check_device_status(DEV)
+    for a, b in zip(*((s.o, s.m, s.l) for s in states)):
+        assert torch.equal(a, b)
+    _check(dtb200.finalize_residual(states[1]), O.attention_fp32(*(t.cpu() for t in (q, k, v))), peak=v.abs().max().item() if second == "e4m3" else None)
