@@ -3,6 +3,7 @@
 Tolerance of the path: bf16 output within max-abs 2e-2 and mean-abs 2e-3 of the fp32-softmax oracle
 on the same seeded inputs; padded query rows exactly zero.
 """
+import ctypes
 import os
 
 import numpy as np
@@ -10,6 +11,7 @@ import pytest
 import torch
 
 import dtb200
+from dtb200 import _lib, ops
 from dtb200.inputs import CONFIGS, make_inputs
 from oracle import attn_oracle as O
 
@@ -30,6 +32,12 @@ def _rand(B, H, Sq, Skv, seed=0, gain=1.0, Hkv=None):
     q = (q * torch.rsqrt(q.pow(2).mean(-1, keepdim=True) + 1e-6) * gain).to(torch.bfloat16)
     k = (k * torch.rsqrt(k.pow(2).mean(-1, keepdim=True) + 1e-6)).to(torch.bfloat16)
     return q, k, v.to(torch.bfloat16)
+
+
+def _block_rows(q, k, num_splits):
+    """Query rows of a block of the launch that these tensors lead to."""
+    p = ops._fill_params(q, k, k, None, None, None, None, 0, num_splits, None)
+    return _lib.load().dtb_attn_block_rows(ctypes.byref(p), None, 0)
 
 
 def _check(out, ref, kv_len=None, tol_scale=1.0):
@@ -369,10 +377,9 @@ def test_concurrent_streams_share_nothing_they_should_not():
 
 @pytest.mark.parametrize("pattern", ["rising", "late_spike", "mixed_rows"])
 def test_offsets_that_move_after_the_first_tile(pattern):
-    """The kernel exponentiates the first half of a tile with the offset it already has and only then confirms it
-    against the tile's maximum; here the maximum does outgrow the offset (by more than the 2^8 of slack) in later
-    tiles - in every tile, in a single late one, or only for some rows of a warp - so the speculated half must be
-    thrown away, the accumulator rescaled, and the result still match the oracle."""
+    """The maximum outgrows the offset by more than the 2^8 of slack in later tiles - in every tile, in a single late one, or only
+    for some rows of a warp - so the accumulator has to be rescaled, which may only happen once the P V of the tile before has
+    run.  Kernels with one and with two query tiles stand at different places when they wait for that: both forms run."""
     g = torch.Generator().manual_seed(21)
     S = 1024                                              # 8 key tiles
     u = torch.randn(128, generator=g)
@@ -393,6 +400,11 @@ def test_offsets_that_move_after_the_first_tile(pattern):
     v = torch.randn(1, 2, S, 128, generator=g)
     q, k, v = q.to(torch.bfloat16), k.to(torch.bfloat16), v.to(torch.bfloat16)
     ref = O.attention_fp32(q, k, v)
-    for splits in (1, 2):
+    for splits, rows in ((1, 128), (2, 256)):
+        assert _block_rows(q, k, splits) == rows
         out = dtb200.attention(q.to(DEV), k.to(DEV), v.to(DEV), num_splits=splits)
         _check(out, ref)
+    # the same two heads on every SM: whole 256-row blocks
+    many = [t.to(DEV).repeat(1, 74, 1, 1) for t in (q, k, v)]
+    assert _block_rows(many[0], many[1], 1) == 256
+    _check(dtb200.attention(*many, num_splits=1), ref.repeat(1, 74, 1, 1))

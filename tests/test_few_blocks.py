@@ -1,7 +1,9 @@
-"""Launches of a few dozen query blocks: pieces of 256-row blocks or whole 128-row blocks, by the number of pieces.
+"""Launches of a few dozen query blocks: pieces of 256-row blocks or whole 128-row blocks.
 
-The lines asserted are those of the rule beside ``kSecondPieceTiles`` in ``attn_api.cu``; on the GPU the calls that it gives to
-128-row blocks agree with float32 attention, and with key splits on 256-row blocks, in the layouts that an entry point takes."""
+The lines asserted are those of the rule beside ``kSecondPieceTiles`` in ``attn_api.cu``, a comparison of two modelled times in which
+the one of the pieces has a surcharge where there are more of them than SMs; 1 x 2 x 3328 and 1 x 2 x 6144 stay in pieces by it
+although they are the slower form there.  On the GPU the calls that it gives to 128-row blocks agree with float32 attention, and
+with key splits on 256-row blocks, in the layouts that an entry point takes."""
 import pytest
 import torch
 
@@ -9,7 +11,8 @@ import dtb200
 
 POLICY = [  # B, heads, rows, 128-row blocks?
     (1, 1, 3072, False), (1, 2, 3072, False), (1, 1, 9216, False), (1, 2, 6144, False), (1, 3, 16896, False), (1, 12, 4608, False),
-    (1, 3, 3072, True), (1, 3, 4608, True), (1, 4, 3072, True), (2, 2, 3072, True), (1, 3, 5200, True), (1, 2, 9216, True),
+    (1, 2, 3328, False),
+    (1, 3, 2560, True), (1, 3, 2816, True), (1, 3, 3072, True), (1, 3, 4608, True), (1, 4, 3072, True), (2, 2, 3072, True), (1, 3, 5200, True), (1, 2, 9216, True),
 ]
 
 
