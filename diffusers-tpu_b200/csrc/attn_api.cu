@@ -307,10 +307,15 @@ constexpr int kMinPieceTiles = 4;      // no run shorter than this many key tile
 #endif
 constexpr int kPieceOverheadTiles = DTB_PIECE_OVERHEAD_TILES;
 
-// What it costs more, beside 128-row blocks, where there are more pieces than SMs, so that some SM sweeps two.  Device time,
-// pieces / 128-row blocks: 1 x 3 heads x 4608 rows (14 + 13 key-tile times by the plan, 30 measured) 45.0 / 36.3 us, 1 x 3 x
-// 3072 34.3 / 26.1, 1 x 4 x 3072 36.4 / 26.2, 1 x 3 x 5200 53.3 / 43.0, 1 x 2 x 9216 85.1 / 74.3; with fewer pieces the plan
-// holds: 1 x 1 x 3072 19.2 / 25.8, 1 x 2 x 3072 22.7 / 26.1, 1 x 1 x 9216 51.6 / 64.8.
+// Taken on top, beside 128-row blocks, where there are more pieces than SMs, so that some SM sweeps two.  An empirical
+// correction, not a cost that was measured by itself: the least that moves 1 x 3 x 3072.  On 148 SMs it moves some of the
+// launches of 25 to 73 query blocks.  Device time in short loops, pieces / 128-row blocks:
+//   moved: 1 x 3 heads x 2560 rows (30 query blocks, 170 pieces) 31.3 / 21.5 us, 1 x 3 x 2816 (33, 174) 33.2 / 22.7, 1 x 3 x 3072
+//   (36, 176) 34.6 / 24.2, 1 x 4 x 3072 (48, 188) 36.5 / 24.4, 1 x 3 x 4608 (54, 196) 44.7 / 33.3, 1 x 3 x 5200 (63, 207) 52.0 /
+//   37.7, 1 x 2 x 9216 (72, 216) 78.0 / 65.4; with K and V of its own for each query block 1 x 73 x 256 against 9088 keys 93.1 / 79.2
+//   not moved, no more pieces than SMs: 1 x 1 x 3072 (72 pieces) 18.9 / 23.6, 1 x 2 x 3072 (144) 23.1 / 24.0
+//   not moved, the plan far enough ahead: 1 x 1 x 9216 (180) 51.0 / 58.7
+//   not moved, though slower in pieces: 1 x 2 x 3328 (168) 31.8 / 25.8, 1 x 2 x 6144 (192) 48.1 / 41.7
 constexpr int kSecondPieceTiles = 3;
 
 // Key-tile times that a block costs beyond its key tiles: launch, pipeline fill and drain, epilogue.
@@ -318,7 +323,7 @@ constexpr int kBlockOverheadTiles = 5;
 
 // Key tiles of the longest walk of a query block, as far as the static shape says: a block-sparse call visits no more
 // than its table is wide.  (Less than four is taken as four, from where a single round goes to 128-row blocks: it is
-// faster there at two tiles already, 74 / 148 blocks 10.6 / 9.4 us.)
+// faster there at two tiles already, 74 / 148 blocks 9.4 / 8.6 us.)
 int key_tiles(const dtb_attn_params* p, const dtb_block_table* tb) {
   const int n = (p->Skv + kBlockN - 1) / kBlockN;
   return tb != nullptr ? std::min(n, std::max(tb->width, 4)) : n;
@@ -332,12 +337,12 @@ long long plain_time(const dtb_attn_params* p, int sms, int rows, long long n) {
 }
 
 // Whether `time` is worse than a launch of 128-row blocks.  Those read K and V once per 128 rows instead of once per
-// 256, which is paid for out of the margin.  Measured, 256-row blocks against 128-row ones, device time:
-//   one round each: 54 / 108 blocks x 18 tiles 31.7 / 21.6 us; 72 / 144 x 36 57.4 / 41.8; 96 / 144 x 132 219 / 159
-//   two rounds against three: 198 / 396 x 132 420 / 410 us in a loop of half a second, under the power limit; 216 / 432 x
-//   36 125 / 124, a model ratio of 0.84, left out
-//   the same with few tiles, as under a narrow table (with P written over S): 222 / 444 x 6 34.0 / 38.1 us, x 12 53.4 / 55.0, x 24 90.0 / 88.0
-//   one against two: 108 / 216 x 36 62.6 / 74.6 us
+// 256, which is paid for out of the margin.  Measured, 256-row blocks against 128-row ones, device time in loops of half a
+// second (the long walks under the power limit):
+//   one round each: 54 / 108 blocks x 18 tiles 31.3 / 20.3 us; 72 / 144 x 36 56.5 / 39.1; 96 / 144 x 132 213 / 151
+//   two rounds against three: 198 / 396 x 132 408 / 381 us; 216 / 432 x 36 122 / 117, a model ratio of 0.84, left out
+//   the same with few tiles, as under a narrow table: 222 / 444 x 6 31.3 / 35.6 us, x 12 49.1 / 50.9, x 24 88.2 / 86.5
+//   one against two: 108 / 216 x 36 61.3 / 69.0 us
 bool solo_beats(const dtb_attn_params* p, int sms, int n, long long time) {
   return 5 * plain_time(p, sms, kBlockM, n) < 4 * time;
 }

@@ -27,11 +27,13 @@
 //   * P_t(j) V_j is issued after the group's arrivals on p_lo and p_hi.
 // Q K^T and P V touch disjoint columns, so the two issuers need no order between them.  They are two warps because a
 // warp does not get past a group of MMAs before the tensor pipe has taken them up: with both kinds in one warp, each wait
-// between two groups is idle time of the pipe (2 x 24 x 16896 rows: 5100 us, 4965 with two warps).
+// between two groups is idle time of the pipe (2 x 24 x 16896 rows, when the first half of P was still exponentiated ahead of
+// the maximum: 5100 us in a burst, 4965 with two warps).  A slot of the ring is committed to only where the producer reloads it.
 //
 // What bounds it: the chain S -> registers -> next Q K^T -> S, twice per key tile, and the MUFU unit's 2048 cycles of
-// exponentials per key tile beside 2048 of tensor pipe.  Measured per call with P over S and one issuer / so, 2 x 24
-// heads: 16896 rows 4888 / 4710 us, 4608 rows 387 / 371, E4M3 scores 4850 / 4550.
+// exponentials per key tile beside 2048 of tensor pipe.  Measured per call with P over S and one issuer / so, 2 x 24 heads, in
+// bursts of 8 ms and in loops of 0.4 s (power limit): 16896 rows 5055 / 4923 and 5599 / 5437 us, 4608 rows 393 / 376 and 429 /
+// 412, E4M3 scores with their casts at 16896 rows 4869 / 4496 and 5265 / 4948.
 #pragma once
 
 #include "ptx.cuh"
@@ -149,11 +151,11 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const 
 // of 64 keys, each published on its own mbarrier so the PV MMA of the first half runs while the second half is still
 // being exponentiated.  wait_pv() returns when the P V of the group's tile before has run; it stands in front of
 // the exponentials, so that the first 32 probabilities can be stored under those of the next 32.  (Behind the first 64, 2 x 24
-// x 4608 rows: online 371 -> 393 us, a bounded call with its smoothing and norms 464 -> 478.)  With two query tiles it also
-// stands in front of the maximum (kWaitFirst: E4M3 scores 2 x 24 x 16896 4890 us, 5040 behind it; 2 x 24 x 4608 412, 415);
-// with one, where loads set the pace, behind it (333 queries against 16731 keys 158 us, 166 in front).  Returns false when a
-// wait ran out.  Exponentiating the first half before the maximum is known, which paid while the next Q K^T waited for P,
-// costs 6% now (371 -> 394 us).
+// x 4608 rows: online 371 -> 393 us in bursts, a bounded call with its smoothing and norms 464 -> 478 in loops of 0.4 s.)  With
+// two query tiles it also stands in front of the maximum (kWaitFirst; 2 x 24 x 16896 in loops of 0.4 s: 5437 us, 5594 behind it,
+// with E4M3 scores and casts 4948 and 5046); with one, behind it, which makes no difference (333 queries against 16731 keys
+// 152 us, 151 in front).  Returns false when a wait ran out.  Exponentiating the first half before the maximum is known, which
+// paid while the next Q K^T waited for P, costs 6% now (371 -> 394 us in bursts), and more where offsets move.
 // ---------------------------------------------------------------------------
 template <bool kFixedM, bool kWaitFirst, class WaitPv>
 __device__ __forceinline__ bool softmax_tile(uint32_t s_tmem, uint32_t p_tmem, uint32_t o_tmem, float scale_log2, int valid_cols,
@@ -426,8 +428,7 @@ __device__ __forceinline__ void attn_fwd_body(const AttnKernelParams& p, const P
     bool ok = true;
 
     // The issuing regions are entered through elect.sync rather than `lane == 0`: with the same instructions inside,
-    // a call on the 1024-pixel image shape takes 399 us against 413 us.  Everything this warp does between two MMA
-    // instructions is idle time of the tensor pipe, so the code the compiler emits around them matters.
+    // a call on the 1024-pixel image shape takes 412 us against 422 in loops of 0.4 s, one on the 2048-pixel shape 5437 against 5481.
     auto issue_qk = [&](int t, int slot) {
       if (elect_one()) {
         const uint64_t a0 = q_desc0 + static_cast<uint64_t>((t * kTileBytes) >> 4);

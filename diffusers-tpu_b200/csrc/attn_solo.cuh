@@ -14,8 +14,8 @@
 //
 // A kernel of its own rather than a case of the other: the two-tile kernel's loop is sensitive to its neighbourhood,
 // and as a template parameter of that body this form cost long sequences 2%.
-// Measured, 256-row blocks -> this: 1 x 6 heads x 2304 rows (54 -> 108 blocks) 31.7 -> 21.6 us; 2 x 24 heads x 333
-// queries against 16731 keys (96 blocks, a third of their rows empty -> 144 blocks) 219 -> 159 us.
+// Measured in loops of half a second, 256-row blocks -> this: 1 x 6 heads x 2304 rows (54 -> 108 blocks) 31.3 -> 20.3 us; 2 x 24
+// heads x 333 queries against 16731 keys (96 blocks, a third of their rows empty -> 144 blocks) 213 -> 151 us.
 #pragma once
 
 #include "attn_kernel.cuh"
